@@ -1,0 +1,49 @@
+"""The tile raster's batch edges: a warp processes the triangles that touch its
+pixels 32 at a time and queues their fragments 64 at a time, so stacks of
+triangles around those counts, over frames that end inside a tile, a micro-tile
+and a pixel group, against the oracle. Small triangles and ones wider than 64
+pixels (whose edge functions need 64 bits) alternate."""
+import numpy as np
+import pytest
+
+import parity_util as pu
+import vk_order_independent_transparency_gb300 as oit
+
+pytestmark = pytest.mark.gpu
+
+
+def stack(n, W, H, seed, large):
+    """n triangles in clip space, from a pixel up to the frame's size (large:
+    every third one reaches far beyond it)."""
+    rng = np.random.default_rng(seed)
+    v = np.zeros((n, 3, 10), np.float32)
+    centre = rng.uniform(-0.8, 0.8, (n, 1, 2))
+    size = rng.uniform(1.0, 8.0, (n, 1, 1)) * 2.0 / np.array([W, H])
+    if large:
+        size[::3] = 6.0 + 200.0 / np.array([W, H])
+    v[:, :, :2] = centre + size * rng.uniform(-1.0, 1.0, (n, 3, 2))
+    v[:, :, 2] = rng.uniform(0.05, 0.95, (n, 3))
+    v[:, :, 3:6] = rng.normal(size=(n, 3, 3))
+    v[:, :, 6:] = rng.random((n, 1, 4))
+    return v.reshape(-1, 10), np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+
+
+def scene_data():
+    sd = oit.OitSceneData()
+    for j in range(4):
+        sd.proj_view_matrix[5 * j] = 1.0
+        sd.view_matrix[5 * j] = 1.0
+    return sd
+
+
+@pytest.mark.parametrize('n,W,H,percent', [(1, 8, 4, 100), (31, 9, 5, 100), (32, 17, 16, 100), (33, 7, 3, 60),
+                                           (64, 16, 17, 100), (65, 33, 21, 50), (161, 24, 9, 75)])
+@pytest.mark.parametrize('aa', [oit.OIT_AA_NONE, oit.OIT_AA_MSAA_8X, oit.OIT_AA_SSAA_4X])
+@pytest.mark.parametrize('alg', range(7))
+def test_stacked_triangles(engine, alg, aa, n, W, H, percent):
+    L = 4
+    v, i = stack(n, W, H, 7 * n + W, large=n % 2 == 1)
+    kw = dict(oit_layers=L, nodes_per_pixel=200, aa_type=aa, weighted_precision=oit.OIT_WEIGHTED_FP32)
+    g = pu.render_gpu(alg, W, H, v, i, 1, scene_data(), percent, **kw)
+    o = pu.render_oracle(alg, W, H, v, i, 1, scene_data(), percent, **kw)
+    pu.check_pair(alg, g, o, W, H, L, aa)

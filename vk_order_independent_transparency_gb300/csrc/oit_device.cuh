@@ -88,14 +88,19 @@ __device__ __forceinline__ float to_float(long long v) { return __ll2float_rn(v)
 __device__ __forceinline__ float to_float(int v) { return __int2float_rn(v); }
 
 // Window depth at the edge values (screen-linear interpolation), clamped to [0,1].
-template <typename E>
-__device__ __forceinline__ float depth_at(const float4& zc, const EdgesT<E>& e) {
-  const float b1 = __fmul_rn(to_float(e.e1), zc.w);
-  const float b2 = __fmul_rn(to_float(e.e2), zc.w);
+// (zc: TriSetup's; e1, e2: the edge values as floats)
+__device__ __forceinline__ float depth_from(const float4& zc, float e1, float e2) {
+  const float b1 = __fmul_rn(e1, zc.w);
+  const float b2 = __fmul_rn(e2, zc.w);
   float z = __fmaf_rn(b2, zc.z, __fmaf_rn(b1, zc.y, zc.x));
   z = (z > 0.0f) ? z : 0.0f;
   z = (z < 1.0f) ? z : 1.0f;
   return z;
+}
+
+template <typename E>
+__device__ __forceinline__ float depth_at(const float4& zc, const EdgesT<E>& e) {
+  return depth_from(zc, to_float(e.e1), to_float(e.e2));
 }
 
 // Exact sRGB8 quantisation tables (gen_srgb_tables.py).
@@ -126,12 +131,12 @@ struct Shade {
   float r, g, b, view_z;
 };
 
-template <typename E>
-__device__ __forceinline__ Shade shade(const TriSetup& T, const EdgesT<E>& e, const TriPersp* P) {
+// (e0, e1, e2: the edge values as floats)
+__device__ __forceinline__ Shade shade_at(const TriSetup& T, float e0, float e1, float e2, const TriPersp* P) {
   const float inv_area = T.zc.w;
-  const float b0 = __fmul_rn(to_float(e.e0), inv_area);
-  const float b1 = __fmul_rn(to_float(e.e1), inv_area);
-  const float b2 = __fmul_rn(to_float(e.e2), inv_area);
+  const float b0 = __fmul_rn(e0, inv_area);
+  const float b1 = __fmul_rn(e1, inv_area);
+  const float b2 = __fmul_rn(e2, inv_area);
   const float4 n0 = T.n0, n1 = T.n1, n2 = T.n2;
   const float nx = __fmaf_rn(b2, n2.x, __fmaf_rn(b1, n1.x, __fmul_rn(b0, n0.x)));
   const float ny = __fmaf_rn(b2, n2.y, __fmaf_rn(b1, n1.y, __fmul_rn(b0, n0.y)));
@@ -152,6 +157,11 @@ __device__ __forceinline__ Shade shade(const TriSetup& T, const EdgesT<E>& e, co
     s.view_z = __fdiv_rn(num, den);
   }
   return s;
+}
+
+template <typename E>
+__device__ __forceinline__ Shade shade(const TriSetup& T, const EdgesT<E>& e, const TriPersp* P) {
+  return shade_at(T, to_float(e.e0), to_float(e.e1), to_float(e.e2), P);
 }
 
 __device__ __forceinline__ uint32_t pack_rgba8(const Shade& s, uint32_t alpha_code) {
