@@ -3,9 +3,8 @@
 // One warp per 8x4 micro-tile of a 16x16 tile, one lane per pixel. Each warp
 // walks its tile's triangle list (primitive order, from the bins), collects the
 // triangles whose bbox touches the micro-tile (the hits) and processes them 32
-// at a time: one lane per hit prepares its edge equations, one lane per (hit,
-// pixel) pair tests coverage, one lane per covered fragment shades it, and the
-// pixel's owner lane runs the algorithm's fragment body (the COLOR/DEPTH shader
+// at a time: one lane per hit prepares its edge equations and finds the pixels
+// it covers, one lane per covered pixel shades a fragment, and the pixel's owner lane runs the algorithm's fragment body (the COLOR/DEPTH shader
 // of the reference) on that pixel's state, so every pixel sees its fragments in
 // primitive order -- the order the reference's hardware blender guarantees for
 // tail blending and the order ordered interlock guarantees for its critical
@@ -80,8 +79,8 @@ struct SimplePolicy {
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = false;
   static __host__ __device__ size_t smem_bytes_per_warp(int, int, int = 0) { return 0; }
-  // the colours that tail blending takes
-  static __host__ __device__ int payload_bytes(int tail, int) { return tail ? 16 : 0; }
+  // the colours and coverage that tail blending takes
+  static __host__ __device__ int payload_bytes(int tail, int) { return tail ? 20 : 0; }
   uint32_t count;
   uint32_t eaux;
   __device__ void init(const RasterParams& p, void*, int, int sample, uint32_t pixel) {
@@ -679,11 +678,10 @@ __device__ __forceinline__ bool lane_in_bbox(uint2 bb, const WarpTile& w) {
 //        dE1/dy} per pixel, where E = 2 e + top_left - 1 for the edge value e
 //        (so a sample is inside when no E is negative, and e = (E + 1) >> 1)
 //        and E2 = sum - E0 - E1 (the edge values add up to twice the area);
-//  hit   the pairs of a hit: number of the first (bits 0-10), x and y of bbox ∩
-//        the warp's pixels relative to the first pixel (bits 11-13, 14-15), its
-//        width (bits 16-19), ceil(256 / width) (bits 20-28), bit 31: not
-//        small; and the record's flags word;
-//  ent   queued fragments: hit (bits 0-4), owner lane (bits 8-12), coverage
+//  hit   the hits that cover a pixel: number of the first covered one (bits
+//        0-10), record (bits 11-15), alpha code (bits 16-23), bit 31: not
+//        small; and the covered pixels, one bit per owner lane;
+//  ent   queued fragments: record (bits 0-4), owner lane (bits 8-12), coverage
 //        (bits 16-23); depth;
 //  mine  per 32 queued fragments and lane: the fragments of the lane's pixel;
 //  ring  triangles collected by the walk;
@@ -697,9 +695,19 @@ struct WarpStage {
 };
 __host__ __device__ constexpr size_t warp_stage_bytes(int payload) { return sizeof(WarpStage) + (size_t)kQueue * payload; }
 
-// ceil(256 / d) for 1 <= d <= 8: r * it >> 8 is r / d for r < 32
-__device__ __forceinline__ uint32_t recip8(int d) {
-  return 32u + (((d <= 4 ? 0x203660E0u >> (8 * (d - 1)) : 0x00050B14u >> (8 * (d - 5)))) & 255u);
+// Position of set bit n (0 = the lowest) of m; n < popc(m).
+__device__ __forceinline__ int nth_bit(uint32_t m, uint32_t n) {
+  int pos = 0;
+#pragma unroll
+  for (int w = 16; w >= 1; w >>= 1) {
+    const uint32_t c = (uint32_t)__popc(m & ((1u << w) - 1u));
+    if (n >= c) {
+      n -= c;
+      m >>= w;
+      pos += w;
+    }
+  }
+  return pos;
 }
 
 // Sample s of SSN in 1/256 pixel, s a run-time value.
@@ -711,17 +719,20 @@ __device__ __forceinline__ int2 sample_pos_at(int s) {
 
 // S: samples each lane evaluates (MSAA coverage); SSN: samples mapped to
 // lanes (sample shading, S = 1 then).
-// The pass is bound by instruction issue (77% issue-active at 1920x1080 with
+// The pass is bound by instruction issue (77-82% issue-active at 1920x1080 with
 // 4096 spheres, WBOIT), so the work is laid out to fill a warp's lanes at each
-// step: 32 hits are prepared at once, 32 (hit, pixel) pairs tested at once,
-// each with five integer operations for its edge values, and 32 fragments
-// shaded at once; what a fragment's algorithm computes from the fragment alone
-// (its weight, its record, its list node) is done by the lane that shaded it.
-// Against hits processed per 32 list entries with the edge functions evaluated
-// from the vertices, whole frames: WBOIT 3840x2160, 16384 spheres 6.84 -> 4.60
-// ms; Interlock 2560x1440 8x MSAA 6.30 -> 4.31 ms; linked list 640x480 215 ->
-// 156 us; Loop32 1001x563 4x sample shading 738 -> 522 us; Loop64 1920x1080
-// with opaque objects 575 -> 485 us.
+// step: 32 hits are prepared at once, each finding the pixels it covers by 32
+// sign tests of five integer operations (a triangle of 6 pixels has a bbox of
+// 26, so testing (hit, bbox pixel) pairs one per lane is four to six tests per
+// fragment, each with the finding of its hit and pixel around it), and 32
+// fragments are shaded at once; what a fragment's algorithm computes from the
+// fragment alone (its weight, its record, its list node) is done by the lane
+// that shaded it. Whole frames with bbox pairs, then with covered pixels: WBOIT
+// 3840x2160, 16384 spheres 4.60 -> 3.32 ms; Interlock 2560x1440 8x MSAA 4.31 ->
+// 3.63 ms; Loop32 1001x563 4x sample shading 522 -> 391 us; Spinlock 800x512
+// 327 -> 288 us; linked list 640x480 156 -> 137 us; 24-view batch 4.78 -> 4.31
+// ms. (With hits processed per 32 list entries and the edge functions evaluated
+// from the vertices: 6.84 ms, 6.30 ms, 738 us, 420 us, 215 us, 6.18 ms.)
 // The warps of a tile work independently (each walks the tile's list for its
 // own micro-tile), so a CTA holds kRasterWarpsPerBlock of them: a CTA's
 // resources are released when its slowest warp is done, and micro-tiles of
@@ -766,20 +777,34 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
   const TriSetup* __restrict__ setup = reinterpret_cast<const TriSetup*>(p.setup);
   const TriPersp* __restrict__ persp = reinterpret_cast<const TriPersp*>(p.persp);
   const uint32_t lt = (1u << w.lane) - 1u;
+  // owner lanes whose pixel exists, and those of the pixels in a bbox
+  const uint32_t lanes = __ballot_sync(kFull, w.valid);
+  auto bbox_lanes = [&](int bx0, int by0, int bx1, int by1) {
+    const int x0 = max(bx0 - w.rx0, 0), x1 = min(bx1 - w.rx0, M::kW - 1);
+    const int y0 = max(by0 - w.ry0, 0), y1 = min(by1 - w.ry0, M::kH - 1);
+    uint32_t m = 0;
+#pragma unroll
+    for (int y = 0; y < M::kH; ++y)
+      if (y >= y0 && y <= y1 && x0 <= x1) m |= ((2u << x1) - (1u << x0)) << (y * M::kW);
+    uint32_t all = m;
+#pragma unroll
+    for (int i = 1; i < SSN; ++i) all |= m << (i * M::kPix);
+    return all;
+  };
   uint32_t nfrag = 0;  // warp-uniform
   uint32_t got = 0;    // fragments delivered to this lane's pixel
   int qn = 0;          // warp-uniform: queued fragments
-  int qs = 0;          // warp-uniform: queued fragments already shaded
 
 #pragma unroll 1
   for (int pass = 0; pass < Pol::kPasses; ++pass) {
     const bool shading = Pol::kPasses == 1 || pass == Pol::kPasses - 1;
 
-    // Stages ring entries head .. head + nh - 1, one lane per hit; returns the
-    // number of the hit's first pair, and the number of pairs of all hits.
+    // Stages ring entries head .. head + nh - 1, one lane per hit, and finds
+    // the pixels each covers, 32 sign tests a lane (with several samples a
+    // lane, or a large triangle: the pixels it may cover). Returns the number
+    // of the hit's first pixel, and the number of pixels of all hits.
     auto stage = [&](uint32_t head, int nh, int& total) {
-      int n = 0;
-      uint32_t range = 0, flags = 0;
+      uint32_t cover = 0, info = 0;
       if (w.lane < nh) {
         const TriSetup* src = setup + st.ring[(head + w.lane) % kRing];
         TriSetup& dst = st.rec[w.lane];
@@ -789,28 +814,61 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
         cp_async16(&dst.n2, &src->n2);
         const int4 a = __ldg(&src->xy01), b = __ldg(&src->xy2f);
         const int X0 = a.x, Y0 = a.y, X1 = a.z, Y1 = a.w, X2 = b.x, Y2 = b.y;
-        flags = (uint32_t)b.z;
-        // bbox ∩ the warp's pixels, relative to the first one
-        const int x0 = max((min(X0, min(X1, X2)) >> 8) - w.rx0, 0), y0 = max((min(Y0, min(Y1, Y2)) >> 8) - w.ry0, 0);
-        const int x1 = min(max(X0, max(X1, X2)) >> 8, min(w.rx1, p.RW - 1)) - w.rx0;
-        const int y1 = min(max(Y0, max(Y1, Y2)) >> 8, min(w.ry1, p.RH - 1)) - w.ry0;
-        const int wd = x1 - x0 + 1;
-        n = wd * (y1 - y0 + 1) * SSN;
-        range = ((uint32_t)x0 << 11) | ((uint32_t)y0 << 14) | ((uint32_t)wd << 16) | (recip8(wd) << 20);
+        const uint32_t flags = (uint32_t)b.z;
+        info = ((uint32_t)w.lane << 11) | ((flags << 8) & 0xFF0000u);
         if (flags & kFlagSmall) {
           const int t0 = (int)(flags & 1u), t1 = (int)((flags >> 1) & 1u), t2 = (int)((flags >> 2) & 1u);
-          const int A0 = Y1 - Y2, B0 = X2 - X1, A1 = Y2 - Y0, B1 = X0 - X2;
+          const int A0 = (Y1 - Y2) * 512, B0 = (X2 - X1) * 512, A1 = (Y2 - Y0) * 512, B1 = (X0 - X2) * 512;
           const int ox = w.rx0 * 256 + (kCentre ? 128 : 0), oy = w.ry0 * 256 + (kCentre ? 128 : 0);
-          const int e0 = B0 * (oy - Y1) + A0 * (ox - X1), e1 = B1 * (oy - Y2) + A1 * (ox - X2);
-          const int area = (X1 - X0) * (Y2 - Y0) - (Y1 - Y0) * (X2 - X0);
-          dst.xy01 = make_int4(2 * e0 + t0 - 1, 2 * e1 + t1 - 1, 2 * area + t0 + t1 + t2 - 3, b.w);
-          dst.xy2f = make_int4(A0 * 512, B0 * 512, A1 * 512, B1 * 512);
+          const int E0 = 2 * ((X2 - X1) * (oy - Y1) + (Y1 - Y2) * (ox - X1)) + t0 - 1;
+          const int E1 = 2 * ((X0 - X2) * (oy - Y2) + (Y2 - Y0) * (ox - X2)) + t1 - 1;
+          const int sum = 2 * ((X1 - X0) * (Y2 - Y0) - (Y1 - Y0) * (X2 - X0)) + t0 + t1 + t2 - 3;
+          dst.xy01 = make_int4(E0, E1, sum, b.w);
+          dst.xy2f = make_int4(A0, B0, A1, B1);
+          // from the last lane to the first, so that each sign shifts in below the ones before it
+          uint32_t out = 0;
+          if (S == 1) {
+#pragma unroll
+            for (int smp = SSN - 1; smp >= 0; --smp) {
+              int s0 = E0, s1 = E1;
+              if (!kCentre) {
+                const int2 sp = sample_pos<SSN>(smp);
+                s0 += (A0 >> 8) * sp.x + (B0 >> 8) * sp.y;
+                s1 += (A1 >> 8) * sp.x + (B1 >> 8) * sp.y;
+              }
+#pragma unroll
+              for (int y = M::kH - 1; y >= 0; --y)
+#pragma unroll
+                for (int x = M::kW - 1; x >= 0; --x) {
+                  const int e0 = s0 + A0 * x + B0 * y, e1 = s1 + A1 * x + B1 * y;
+                  out = __funnelshift_l((uint32_t)(e0 | e1 | (sum - e0 - e1)), out, 1);
+                }
+            }
+          } else {
+            // the largest value over the pixel's samples (all of them within 16 .. 240)
+            const int A2 = -(A0 + A1), B2 = -(B0 + B1);
+            auto most = [](int A, int B) {
+              return (max(A, 0) >> 8) * 240 + (min(A, 0) >> 8) * 16 + (max(B, 0) >> 8) * 240 + (min(B, 0) >> 8) * 16;
+            };
+            const int s0 = E0 + most(A0, B0), s1 = E1 + most(A1, B1), s2 = sum - E0 - E1 + most(A2, B2);
+#pragma unroll
+            for (int y = M::kH - 1; y >= 0; --y)
+#pragma unroll
+              for (int x = M::kW - 1; x >= 0; --x) {
+                const int e0 = s0 + A0 * x + B0 * y, e1 = s1 + A1 * x + B1 * y, e2 = s2 + A2 * x + B2 * y;
+                out = __funnelshift_l((uint32_t)(e0 | e1 | e2), out, 1);
+              }
+          }
+          cover = ~out & lanes;
         } else {
-          range |= 0x80000000u;
+          info |= 0x80000000u;
           dst.xy01 = a;
           dst.xy2f = b;
+          cover = bbox_lanes(min(X0, min(X1, X2)) >> 8, min(Y0, min(Y1, Y2)) >> 8, max(X0, max(X1, X2)) >> 8,
+                             max(Y0, max(Y1, Y2)) >> 8) & lanes;
         }
       }
+      const int n = __popc(cover);
       int incl = n;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -818,24 +876,20 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
         if (w.lane >= o) incl += y;
       }
       total = __shfl_sync(kFull, incl, 31);
-      if (w.lane < nh) st.hit[w.lane] = make_uint2(range | (uint32_t)(incl - n), flags);
+      const uint32_t some = __ballot_sync(kFull, n > 0);
+      if (n > 0) st.hit[__popc(some & lt)] = make_uint2(info | (uint32_t)(incl - n), cover);
       cp_async_wait_all();
       __syncwarp();
-      return w.lane < nh ? incl - n : 0x40000000;
+      return n > 0 ? incl - n : 0x40000000;
     };
 
-    // Shading of a queued fragment: at the pixel centre, or at its own sample
-    // with sample shading. `alpha` is the record's.
-    auto shade_entry = [&](uint2 e, uint32_t head, Frag& f, Shade& sh, float& alpha) {
-      const int k = (int)(e.x & 31u), owner = (int)((e.x >> 8) & 31u);
-      f.cover = e.x >> 16;
-      f.depth = e.y;
-      const TriSetup& T = st.rec[k];
-      const uint2 h = st.hit[k];
+    // Edge values of hit h, record T at owner lane `owner`'s shading point: its
+    // pixel's centre, or its sample with sample shading. False when a large
+    // triangle does not cover it.
+    auto edges = [&](uint2 h, const TriSetup& T, int owner, float3& v, float& alpha) {
       const int4 a = T.xy01, b = T.xy2f;
       const int pl = M::pix(owner), dx = pl % M::kW, dy = pl / M::kW;
       const int2 sp = SSN > 1 ? sample_pos_at<SSN>(M::sample(owner)) : make_int2(128, 128);
-      float3 v;
       if (!(h.x >> 31)) {
         int e0 = a.x + b.x * dx + b.y * dy, e1 = a.y + b.z * dx + b.w * dy;
         if (!kCentre) {
@@ -845,37 +899,44 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
         const int e2 = a.z - e0 - e1;
         v = make_float3(to_float((e0 + 1) >> 1), to_float((e1 + 1) >> 1), to_float((e2 + 1) >> 1));
         alpha = __int_as_float(a.w);
-      } else {
-        const Edges ed = edges_at<long long>(a, b, (w.rx0 + dx) * 256 + sp.x, (w.ry0 + dy) * 256 + sp.y);
-        v = make_float3(to_float(ed.e0), to_float(ed.e1), to_float(ed.e2));
-        alpha = __int_as_float(b.w);
+        return true;
       }
-      sh = shade_at(T, v.x, v.y, v.z, Pol::kViewZ ? persp + st.ring[(head + k) % kRing] : nullptr);
-      f.packed = Pol::kPack ? pack_rgba8(sh, (h.y >> 8) & 255u) : 0u;
+      const Edges ed = edges_at<long long>(a, b, (w.rx0 + dx) * 256 + sp.x, (w.ry0 + dy) * 256 + sp.y);
+      v = make_float3(to_float(ed.e0), to_float(ed.e1), to_float(ed.e2));
+      alpha = __int_as_float(b.w);
+      return inside(ed, b.z);
     };
 
-    // Direct policies: shades the first `cnt` <= 32 queued fragments, one per
-    // lane, each of which writes its own record, and moves the rest forward.
-    auto drain_direct = [&](uint32_t head, int cnt) {
-      uint32_t node0 = 0;
-      if (Pol::kNodes && w.lane == 0) node0 = atomicAdd(p.counter, (uint32_t)cnt);
-      const bool act = w.lane < cnt;
-      const uint2 e = st.ent[w.lane];
-      const int owner = (int)((e.x >> 8) & 31u);
-      Frag f;
-      Shade sh;
-      float alpha = 0.f;
-      if (act) shade_entry(e, head, f, sh, alpha);
-      const uint32_t lower = act ? st.mine[0][owner] & lt : 0u;  // earlier ones of the same pixel
-      const uint32_t own = st.mine[0][w.lane];                   // this lane's pixel's
+    // Shading of record T from its edge values.
+    auto shade_fragment = [&](uint2 h, uint32_t head, const TriSetup& T, float3 v, Frag& f, Shade& sh) {
+      const int k = (int)((h.x >> 11) & 31u);
+      sh = shade_at(T, v.x, v.y, v.z, Pol::kViewZ ? persp + st.ring[(head + k) % kRing] : nullptr);
+      f.packed = Pol::kPack ? pack_rgba8(sh, (h.x >> 16) & 255u) : 0u;
+    };
+
+    // Direct policies: every active lane holds a shaded fragment and writes its
+    // own record. `lower`: the earlier ones of its pixel, `own`: this lane's
+    // pixel's fragments (one bit per lane that holds one).
+    auto write_direct = [&](bool act, uint32_t am, int owner, const Frag& f, const Shade& sh, float alpha,
+                            uint32_t node0) {
+      if (act) atomicOr(&st.mine[0][owner], 1u << w.lane);
+      __syncwarp();
+      const uint32_t lower = act ? st.mine[0][owner] & lt : 0u;
+      const uint32_t own = st.mine[0][w.lane];
+      __syncwarp();
+      st.mine[0][w.lane] = 0u;
       if constexpr (Pol::kNodes) {
         node0 = __shfl_sync(kFull, node0, 0);
-        const uint32_t before = __shfl_sync(kFull, pol.head, act ? owner : 0);
-        const uint32_t node = node0 + (uint32_t)w.lane + 1u;
+        const uint32_t before = __shfl_sync(kFull, pol.head, owner);
+        const uint32_t node = node0 + (uint32_t)__popc(am & lt) + 1u;
         const bool stored = act && node < p.capacity;
-        if (stored) Pol::write(p, node, lower ? node0 + (32u - (uint32_t)__clz(lower)) : before, f, sh, alpha);
+        // the pixel's last earlier node: its lane's rank among the active ones
+        auto node_of = [&](uint32_t lanes_of) {
+          return node0 + (uint32_t)__popc(am & (0xFFFFFFFFu >> __clz(lanes_of)));
+        };
+        if (stored) Pol::write(p, node, lower ? node_of(lower) : before, f, sh, alpha);
         const uint32_t sm = __ballot_sync(kFull, stored);
-        uint32_t tails = p.tail ? __ballot_sync(kFull, act && !stored) : 0u;
+        uint32_t tails = p.tail ? am & ~sm : 0u;
         while (tails) {  // a full pool: the fragments are tail blended one after the other
           const int j = __ffs(tails) - 1;
           tails &= tails - 1u;
@@ -884,9 +945,9 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
           const uint32_t cover = __shfl_sync(kFull, f.cover, j);
           if (__shfl_sync(kFull, owner, j) == w.lane) tg.tail(c, cover);
         }
-        if (own & sm) pol.head = node0 + (32u - (uint32_t)__clz(own & sm));
+        if (own & sm) pol.head = node_of(own & sm);
       } else if constexpr (Pol::kDirect) {
-        const uint32_t rank = __shfl_sync(kFull, pol.count, act ? owner : 0) + (uint32_t)__popc(lower);
+        const uint32_t rank = __shfl_sync(kFull, pol.count, owner) + (uint32_t)__popc(lower);
         if (act) {
           if (rank < (uint32_t)p.L) {
             const int pl = M::pix(owner);
@@ -894,6 +955,7 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
                        (uint32_t)(w.ry0 + pl / M::kW) * (uint32_t)p.RW + (uint32_t)(w.rx0 + pl % M::kW), f);
           } else if (p.tail) {
             pay.rgba[w.lane] = premult(sh.r, sh.g, sh.b, alpha);
+            pay.packed[w.lane] = f.cover;
           }
         }
         if (p.tail) {
@@ -903,40 +965,19 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
           while (m) {
             const int j = __ffs(m) - 1;
             m &= m - 1u;
-            tg.tail(pay.rgba[j], st.ent[j].x >> 16);
+            tg.tail(pay.rgba[j], pay.packed[j]);
           }
         }
         pol.count += (uint32_t)__popc(own);
       }
       got += (uint32_t)__popc(own);
-      nfrag += (uint32_t)cnt;
-      const uint2 en = st.ent[32 + w.lane];
-      const uint32_t mn = st.mine[1][w.lane];
-      __syncwarp();
-      st.ent[w.lane] = en;
-      st.mine[0][w.lane] = mn;
-      st.mine[1][w.lane] = 0u;
-      qn -= cnt;
+      nfrag += (uint32_t)__popc(am);
       __syncwarp();
     };
 
-    // Queued policies: shades the fragments not shaded yet (their records are
-    // still staged) and, with `feed`, hands every lane its pixel's fragments
-    // in queue order.
-    auto drain_queue = [&](uint32_t head, bool feed) {
-      if (shading) {
-#pragma unroll 1
-        for (int j = qs + w.lane; j < qn; j += 32) {
-          Frag f;
-          Shade sh;
-          float alpha;
-          shade_entry(st.ent[j], head, f, sh, alpha);
-          if constexpr (!Pol::kDirect) Pol::produce(p, pay, j, f, sh, alpha);
-        }
-        __syncwarp();
-      }
-      qs = qn;
-      if (!feed) return;
+    // Queued policies: hands every lane its pixel's fragments in queue order.
+    auto feed = [&]() {
+      __syncwarp();
       unsigned long long m = (unsigned long long)st.mine[0][w.lane] | ((unsigned long long)st.mine[1][w.lane] << 32);
       st.mine[0][w.lane] = 0u;
       st.mine[1][w.lane] = 0u;
@@ -950,107 +991,158 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
         const uint2 e = st.ent[j];
         Frag f;
         f.depth = e.y;
-        f.cover = e.x >> 16;
+        f.cover = S > 1 ? e.x >> 16 : 1u;
         f.packed = shading ? pay.packed[j] : 0u;
         if constexpr (!Pol::kDirect) pol.fragment(p, pass, f, pay, j, tg);
       }
       qn = 0;
-      qs = 0;
       __syncwarp();
     };
 
     walk_pass<(SSN > 1)>(p, w, st.ring, beg, end, [&](uint32_t head, int nh, bool last) {
       int total = 0;
       const int pre = stage(head, nh, total);
-      // The pixels (and samples) of every hit's bbox ∩ the warp's pixels are
-      // numbered hit by hit, row by row; lane g of each group of 32 tests pair
-      // g, reading the owner lane's opaque depth by shuffle. Fragments enter
-      // the queue in lane order, i.e. in primitive order.
+      // The covered pixels of all hits are numbered hit by hit; lane g of each
+      // group of 32 takes number g, so fragments come in primitive order.
       int khi = -1;  // the last hit that starts before this group
+      int qs = qn;   // queued fragments already shaded
 #pragma unroll 1
       for (int base = 0; base < total || last; base += 32) {
         if (!last) {
           const uint32_t rel = (uint32_t)(pre - base);
           const uint32_t starts = __reduce_or_sync(kFull, rel < 32u ? 1u << rel : 0u);
-          const int k = khi + __popc(starts & (lt | (1u << w.lane)));
+          const int j = khi + __popc(starts & (lt | (1u << w.lane)));
           khi += __popc(starts);
-          const int g = base + w.lane;
-          const bool act = g < total;
-          const uint32_t hk = st.hit[k].x;
-          int r = g - (int)(hk & 0x7FFu);
-          const int smp = SSN > 1 ? r & (SSN - 1) : 0;
-          if (SSN > 1) r /= SSN;
-          const int wdt = (int)((hk >> 16) & 0xFu);
-          const int row = (r * (int)((hk >> 20) & 0x1FFu)) >> 8;  // exact r / wdt for 0 <= r < 32, wdt <= 8
-          const int dx = (int)((hk >> 11) & 7u) + r - row * wdt, dy = (int)((hk >> 14) & 3u) + row;
-          const int owner = act ? smp * M::kPix + dy * M::kW + dx : 0;
-          // opaque depth of the pixel's sample s: the owner lane's, or, with
-          // several samples a lane, from memory (they would cost 2 S registers)
-          const uint32_t od = S == 1 ? __shfl_sync(kFull, depth, owner) : 0x3F800000u;
-          const uint32_t* odp = p.depth + (size_t)(w.ry0 + dy) * p.RW + (w.rx0 + dx);
-          auto opaque_depth = [&](int s) {
-            if (S == 1 || !p.has_opaque) return od;
-            return __ldg(odp + (size_t)s * p.P);
-          };
-          uint32_t cover = 0;
-          float zcen = 0.f;
-          if (act) {
-            const TriSetup& T = st.rec[k];
-            const int4 a = T.xy01, b = T.xy2f;
-            const float4 zc = T.zc;
-            if (!(hk >> 31)) {
-              const int E0 = a.x + b.x * dx + b.y * dy, E1 = a.y + b.z * dx + b.w * dy;
-#pragma unroll
-              for (int s = 0; s < S; ++s) {
-                const int2 sp = SSN > 1 ? sample_pos_at<SSN>(smp) : sample_pos<S>(s);
-                int e0 = E0, e1 = E1;
-                if (!kCentre) {
-                  e0 += (b.x >> 8) * sp.x + (b.y >> 8) * sp.y;
-                  e1 += (b.z >> 8) * sp.x + (b.w >> 8) * sp.y;
-                }
-                const int e2 = a.z - e0 - e1;
-                if ((e0 | e1 | e2) >= 0) {
-                  const float z = depth_from(zc, to_float((e1 + 1) >> 1), to_float((e2 + 1) >> 1));
-                  if (__float_as_uint(z) < opaque_depth(s)) cover |= 1u << s;
-                  if (S == 1) zcen = z;
-                }
-              }
-              if (S > 1 && cover) {
-                const int e0 = E0 + (b.x >> 1) + (b.y >> 1), e1 = E1 + (b.z >> 1) + (b.w >> 1);
-                zcen = depth_from(zc, to_float((e1 + 1) >> 1), to_float((a.z - e0 - e1 + 1) >> 1));
-              }
-            } else {
-              const int bxp = (w.rx0 + dx) * 256, byp = (w.ry0 + dy) * 256;
-#pragma unroll 1
-              for (int s = 0; s < S; ++s) {
-                const int2 sp = SSN > 1 ? sample_pos_at<SSN>(smp) : S > 1 ? sample_pos_at<S>(s) : make_int2(128, 128);
-                const Edges e = edges_at<long long>(a, b, bxp + sp.x, byp + sp.y);
-                if (inside(e, b.z)) {
-                  const float z = depth_at(zc, e);
-                  if (__float_as_uint(z) < opaque_depth(s)) cover |= 1u << s;
-                  if (S == 1) zcen = z;
-                }
-              }
-              if (S > 1 && cover) zcen = depth_at(zc, edges_at<long long>(a, b, bxp + 128, byp + 128));
+          const bool act = base + w.lane < total;
+          const uint2 h = st.hit[j];
+          const int k = (int)((h.x >> 11) & 31u);
+          const TriSetup& T = st.rec[k];
+          const int owner = act ? nth_bit(h.y, (uint32_t)(base + w.lane) - (h.x & 0x7FFu)) : w.lane;
+          if constexpr (S == 1) {
+            const uint32_t od = __shfl_sync(kFull, depth, owner);
+            Frag f;
+            f.cover = 1u;
+            float3 v;
+            float alpha = 0.f;
+            bool pass_z = act;
+            if (act) {
+              pass_z = edges(h, T, owner, v, alpha);
+              f.depth = __float_as_uint(depth_from(T.zc, v.y, v.z));
+              pass_z = pass_z && f.depth < od;
             }
+            const uint32_t pm = __ballot_sync(kFull, pass_z);
+            if (pm) {
+              Shade sh;
+              if constexpr (Pol::kDirect) {
+                uint32_t node0 = 0;
+                if (Pol::kNodes && w.lane == 0) node0 = atomicAdd(p.counter, (uint32_t)__popc(pm));
+                if (pass_z) shade_fragment(h, head, T, v, f, sh);
+                write_direct(pass_z, pm, owner, f, sh, alpha, node0);
+              } else {
+                if (pass_z) {
+                  const int e = qn + __popc(pm & lt);
+                  st.ent[e] = make_uint2(0u, f.depth);
+                  atomicOr(&st.mine[e >> 5][owner], 1u << (e & 31));
+                  if (shading) {
+                    shade_fragment(h, head, T, v, f, sh);
+                    Pol::produce(p, pay, e, f, sh, alpha);
+                  }
+                }
+                qn += __popc(pm);
+              }
+            }
+          } else {
+            // coverage of the pixel's samples, then a queue of covered pixels
+            uint32_t cover = 0;
+            float zcen = 0.f;
+            if (act) {
+              const int4 a = T.xy01, b = T.xy2f;
+              const float4 zc = T.zc;
+              const int dx = owner % M::kW, dy = owner / M::kW;
+              const uint32_t* odp = p.depth + (size_t)(w.ry0 + dy) * p.RW + (w.rx0 + dx);
+              // opaque depth, from memory (in the owner lane it would take S registers)
+              auto opaque_depth = [&](int s) { return p.has_opaque ? __ldg(odp + (size_t)s * p.P) : 0x3F800000u; };
+              if (!(h.x >> 31)) {
+                const int E0 = a.x + b.x * dx + b.y * dy, E1 = a.y + b.z * dx + b.w * dy;
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                  const int2 sp = sample_pos<S>(s);
+                  const int e0 = E0 + (b.x >> 8) * sp.x + (b.y >> 8) * sp.y;
+                  const int e1 = E1 + (b.z >> 8) * sp.x + (b.w >> 8) * sp.y;
+                  const int e2 = a.z - e0 - e1;
+                  if ((e0 | e1 | e2) >= 0) {
+                    const float z = depth_from(zc, to_float((e1 + 1) >> 1), to_float((e2 + 1) >> 1));
+                    if (__float_as_uint(z) < opaque_depth(s)) cover |= 1u << s;
+                  }
+                }
+                if (cover) {
+                  const int e0 = E0 + (b.x >> 1) + (b.y >> 1), e1 = E1 + (b.z >> 1) + (b.w >> 1);
+                  zcen = depth_from(zc, to_float((e1 + 1) >> 1), to_float((a.z - e0 - e1 + 1) >> 1));
+                }
+              } else {
+                const int bxp = (w.rx0 + dx) * 256, byp = (w.ry0 + dy) * 256;
+#pragma unroll 1
+                for (int s = 0; s < S; ++s) {
+                  const int2 sp = sample_pos_at<S>(s);
+                  const Edges e = edges_at<long long>(a, b, bxp + sp.x, byp + sp.y);
+                  if (inside(e, b.z) && __float_as_uint(depth_at(zc, e)) < opaque_depth(s)) cover |= 1u << s;
+                }
+                if (cover) zcen = depth_at(zc, edges_at<long long>(a, b, bxp + 128, byp + 128));
+              }
+            }
+            const uint32_t m = __ballot_sync(kFull, cover != 0);
+            if (cover) {
+              const int e = qn + __popc(m & lt);
+              st.ent[e] = make_uint2((uint32_t)j | ((uint32_t)owner << 8) | (cover << 16), __float_as_uint(zcen));
+              if (!Pol::kDirect) atomicOr(&st.mine[e >> 5][owner], 1u << (e & 31));
+            }
+            qn += __popc(m);
+            __syncwarp();
           }
-          const bool has = cover != 0;
-          const uint32_t m = __ballot_sync(kFull, has);
-          if (has) {
-            const int j = qn + __popc(m & lt);
-            st.ent[j] = make_uint2((uint32_t)k | ((uint32_t)owner << 8) | (cover << 16), __float_as_uint(zcen));
-            atomicOr(&st.mine[j >> 5][owner], 1u << (j & 31));
-          }
-          qn += __popc(m);
-          __syncwarp();
         }
         // the next group may add 32 fragments; the next hits replace the records
         const bool done = base + 32 >= total;
-        if constexpr (Pol::kDirect) {
+        if constexpr (S > 1) {
+          // shades the covered pixels
 #pragma unroll 1
-          while (qn >= 32 || (done && qn > 0)) drain_direct(head, min(qn, 32));
-        } else {
-          if (qn > kQueue - 32 || done) drain_queue(head, qn > kQueue - 32 || last);
+          while (shading && qn > qs && (done || qn > kQueue - 32 || (Pol::kDirect && qn >= 32))) {
+            const int e = qs + w.lane;
+            const bool act = e < qn;
+            const uint2 en = st.ent[e % kQueue];
+            const int owner = (int)((en.x >> 8) & 31u);
+            const uint2 h = st.hit[en.x & 31u];
+            const TriSetup& T = st.rec[(h.x >> 11) & 31u];
+            const int cnt = min(qn - qs, 32);
+            uint32_t node0 = 0;
+            if (Pol::kDirect && Pol::kNodes && w.lane == 0) node0 = atomicAdd(p.counter, (uint32_t)cnt);
+            Frag f;
+            Shade sh;
+            float alpha = 0.f;
+            if (act) {
+              float3 v;
+              f.cover = (en.x >> 16) & 255u;
+              f.depth = en.y;
+              edges(h, T, owner, v, alpha);
+              shade_fragment(h, head, T, v, f, sh);
+            }
+            if constexpr (Pol::kDirect) {
+              write_direct(act, cnt == 32 ? kFull : (1u << cnt) - 1u, owner, f, sh, alpha, node0);
+              const uint2 nx = st.ent[32 + w.lane];
+              __syncwarp();
+              st.ent[w.lane] = nx;
+              qn -= cnt;
+              __syncwarp();
+            } else {
+              if (act) Pol::produce(p, pay, e, f, sh, alpha);
+              qs += cnt;
+            }
+          }
+        }
+        if constexpr (!Pol::kDirect) {
+          if (last || qn > kQueue - 32) {
+            feed();
+            qs = 0;
+          }
         }
         if (last) break;
       }
