@@ -8,8 +8,7 @@ so that the CPU oracle and the CUDA kernels pick the same code for every input:
 
   thr[k]    (k = 0..254) smallest float c with enc(c)*255 >= k + 0.5,
             enc evaluated in double; thr[255] = 3e38 sentinel.
-  bucket[i] (i = 0..4095) code of c = i/4096, so that
-            code(c) = bucket[floor(c*4096)] + (c >= thr[bucket[...]]).
+            code(c) = the number of thresholds <= c.
   dec[k]    linear value of sRGB code k, rounded to float.
 
 Run: python gen_srgb_tables.py > srgb_tables.inc
@@ -48,17 +47,6 @@ def thresholds():
     return out
 
 
-def code_of(c, thr):
-    lo, hi = 0, 255
-    while lo < hi:
-        mid = (lo + hi) >> 1
-        if c >= thr[mid]:
-            lo = mid + 1
-        else:
-            hi = mid
-    return lo
-
-
 def decode(k):
     s = k / 255.0
     return s / 12.92 if s < 0.04045 else math.pow((s + 0.055) / 1.055, 2.4)
@@ -66,7 +54,6 @@ def decode(k):
 
 def main(out=sys.stdout):
     thr = thresholds()
-    bucket = [code_of(b2f(f2b(i / 4096.0)), thr) for i in range(4096)]
     dec = [b2f(f2b(decode(k))) for k in range(256)]
     w = out.write
     w('// Generated by gen_srgb_tables.py; do not edit.\n')
@@ -74,10 +61,6 @@ def main(out=sys.stdout):
     for k in range(255):
         w('  %s, \\\n' % (float.hex(thr[k]) + 'f'))
     w('  3.0e38f }\n')
-    w('#define OIT_SRGB_BUCKET_INIT { \\\n')
-    for i in range(0, 4096, 32):
-        w('  ' + ', '.join(str(v) for v in bucket[i:i + 32]) + ', \\\n')
-    w('}\n')
     w('#define OIT_SRGB_DEC_INIT { \\\n')
     for k in range(256):
         w('  %s, \\\n' % (float.hex(dec[k]) + 'f'))
