@@ -47,3 +47,28 @@ def test_stacked_triangles(engine, alg, aa, n, W, H, percent):
     g = pu.render_gpu(alg, W, H, v, i, 1, scene_data(), percent, **kw)
     o = pu.render_oracle(alg, W, H, v, i, 1, scene_data(), percent, **kw)
     pu.check_pair(alg, g, o, W, H, L, aa)
+
+
+@pytest.mark.parametrize('aa', [oit.OIT_AA_NONE, oit.OIT_AA_MSAA_4X])
+@pytest.mark.parametrize('cuts', [(0, 90), (0, 1, 90), (0, 0, 45, 90), (0, 90, 90)])
+def test_opaque_draws_accumulate(engine, aa, cuts):
+    """Opaque draws one after the other (the first one clears, an empty one
+    only clears) leave what one draw of all triangles leaves."""
+    W, H = 37, 19
+    v, i = stack(90, W, H, 5, large=True)
+    mesh = oit.DeviceMesh(v, i)
+
+    def targets(bounds):
+        with oit.Renderer(oit.make_state(oit.OIT_SIMPLE, W, H, aa_type=aa)) as r:
+            r.update_scene(scene_data())
+            for _ in range(2):  # the second frame finds the first one's targets
+                r.begin_frame()
+                r.clear_transparent()
+                for a, b in zip(bounds, bounds[1:]):
+                    r.draw_opaque(mesh, a, b - a)
+                r.draw_transparent_color(mesh, 0, 0)
+                r.composite()
+            return r.read_buffer(oit.OIT_BUF_DEPTH), r.read_buffer(oit.OIT_BUF_OPAQUE_COLOR), r.output()
+
+    for a, b in zip(targets(cuts), targets((0, 90))):
+        np.testing.assert_array_equal(a, b)

@@ -118,6 +118,7 @@ struct oit_context {
   size_t tri_cap = 0, pair_cap = 0;
   uint32_t bin_tris = 0, bin_opaque_from = 0;  // the last binned draw: triangles, first opaque one
   bool opaque_valid = false;
+  bool opaque_started = false;  // the frame's opaque targets are written (else its first opaque pass clears them)
   bool color_valid = false;
   int raster_wpsm = 0;  // RasterParams::warps_per_sm of this context's transparent rasters
   cudaStream_t last_stream = nullptr;
@@ -550,6 +551,7 @@ struct oit_context {
   int begin_frame(cudaStream_t s) {
     last_stream = s;
     opaque_valid = false;
+    opaque_started = false;
     color_valid = false;
     return OIT_OK;
   }
@@ -564,27 +566,30 @@ struct oit_context {
     return OIT_OK;
   }
 
+  // The first opaque draw of a frame starts from the clear values itself
+  // (opaque_fresh) and writes every pixel; an empty one only clears.
   int draw_opaque(const oit::MeshRef& mesh, uint32_t first, uint32_t count, cudaStream_t s) {
     last_stream = s;
-    int r = clear_opaque_targets(s);
+    int r = ensure_opaque_buffers();
     if (r != OIT_OK) return r;
-    if (!count) return OIT_OK;
+    opaque_valid = true;
+    if (!count) return clear_opaque_targets(s);
     cudaEvent_t t0 = prof_begin(s);
     r = bin(mesh, first, count, 0u, s);
-    if (r != OIT_OK) return r;
+    if (r != OIT_OK) {
+      clear_opaque_targets(s);
+      return r;
+    }
     prof_end(OIT_PROF_OPAQUE_BIN, t0, s);
     return raster_opaque(s);
   }
 
   int clear_opaque_targets(cudaStream_t s) {
-    int r = ensure_opaque_buffers();
-    if (r != OIT_OK) return r;
-    if (!opaque_valid) {
-      OIT_TRY_CUDA(oit::launch_fill_u32(depth.as<uint32_t>(), 0x3F800000u, (size_t)S * P, s), "fill");
-      OIT_TRY_CUDA(oit::launch_fill_f4(opaque_color.as<float4>(), background, (size_t)S * P, s), "fill");
-      launches += 2;
-      opaque_valid = true;
-    }
+    if (opaque_started) return OIT_OK;
+    OIT_TRY_CUDA(oit::launch_fill_u32(depth.as<uint32_t>(), 0x3F800000u, (size_t)S * P, s), "fill");
+    OIT_TRY_CUDA(oit::launch_fill_f4(opaque_color.as<float4>(), background, (size_t)S * P, s), "fill");
+    launches += 2;
+    opaque_started = true;
     return OIT_OK;
   }
 
@@ -592,6 +597,7 @@ struct oit_context {
     oit::RasterParams p = raster_params(0);
     p.S = S;    // the opaque pass always tests every sample of a pixel
     p.ssn = 1;
+    p.opaque_fresh = opaque_started ? 0 : 1;
     return p;
   }
 
@@ -600,6 +606,7 @@ struct oit_context {
     cudaEvent_t t1 = prof_begin(s);
     const int r = raster(oit::Alg::Opaque, p, s);
     prof_end(OIT_PROF_OPAQUE_RASTER, t1, s);
+    if (r == OIT_OK) opaque_started = true;
     return r;
   }
 
@@ -726,8 +733,9 @@ struct oit_context {
     const uint32_t nt = num_transparent * tpo, total_tris = num_objects * tpo;
     int r = begin_frame(s);
     if (r == OIT_OK) r = clear_transparent(s);
-    if (r == OIT_OK && num_opaque > 0) r = clear_opaque_targets(s);
+    if (r == OIT_OK && num_opaque > 0) r = ensure_opaque_buffers();
     if (r != OIT_OK) return r;
+    opaque_valid = num_opaque > 0;
     cudaEvent_t t0 = prof_begin(s);
     r = bin(mesh, 0, total_tris, nt, s);
     if (r != OIT_OK) return r;

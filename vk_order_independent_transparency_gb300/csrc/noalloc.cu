@@ -183,10 +183,6 @@ extern "C" int oit_render_frame_noalloc(const oit_state* st, const oit_scene_dat
   std::memcpy(scene_words + 16, scene->view_matrix, 16 * sizeof(float));
   NOALLOC_TRY(cudaMemcpyAsync(scene_dev, scene_words, sizeof(scene_words), cudaMemcpyHostToDevice, s));
   const float4 bg = make_float4(0.2f, 0.2f, 0.2f, 0.2f);  // oitRender.cpp:90
-  if (opaque) {
-    NOALLOC_TRY(launch_fill_u32(depth, 0x3F800000u, (size_t)S * P, s));
-    NOALLOC_TRY(launch_fill_f4(opaque_color, bg, (size_t)S * P, s));
-  }
   SetupParams sp{};
   sp.vertices = mesh->vertices_device;
   sp.indices = mesh->indices_device;
@@ -243,6 +239,7 @@ extern "C" int oit_render_frame_noalloc(const oit_state* st, const oit_scene_dat
   p.depth = depth;
   p.opaque_color = opaque_color;
   p.has_opaque = opaque ? 1 : 0;
+  p.opaque_fresh = 1;
   p.background = bg;
   p.color = color;
   p.color_half = half_color ? 1 : 0;

@@ -124,6 +124,7 @@ struct RasterParams {
   uint32_t* depth;               // [S][P] opaque depth (read by transparent passes)
   float4* opaque_color;          // [S][P]
   int has_opaque;                // 0: depth 1.0 and background colour everywhere
+  int opaque_fresh;              // opaque pass: start from depth 1.0 and background colour and write every pixel
   float4 background;
   float4* color;                 // [ssn][P] colour target after tail blend (sample average unless sample shading)
   int color_half;                // the colour target holds four halves per element

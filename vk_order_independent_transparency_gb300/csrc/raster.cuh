@@ -663,11 +663,6 @@ __device__ __forceinline__ void walk_pass(const RasterParams& p, const WarpTile&
   }
 }
 
-__device__ __forceinline__ bool lane_in_bbox(uint2 bb, const WarpTile& w) {
-  return w.valid && w.px >= (int)(bb.x & 0xFFFF) && w.px <= (int)(bb.y & 0xFFFF) && w.py >= (int)(bb.x >> 16) &&
-         w.py <= (int)((bb.y >> 16) & 0x7FFF);
-}
-
 // ---------------------------------------------------------------------------
 // Transparent COLOR (+DEPTH) pass.
 // ---------------------------------------------------------------------------
@@ -715,6 +710,116 @@ template <int SSN>
 __device__ __forceinline__ int2 sample_pos_at(int s) {
   const uint32_t x = SSN == 4 ? 0xA2E6u : 0xFB135D79u, y = SSN == 4 ? 0xEA62u : 0x1F7D39B5u;
   return make_int2((int)((x >> (4 * s)) & 15u) << 4, (int)((y >> (4 * s)) & 15u) << 4);
+}
+
+// The owner lanes (bits) of the warp's pixels in a bbox.
+template <int SSN>
+__device__ __forceinline__ uint32_t bbox_lanes(const WarpTile& w, int bx0, int by0, int bx1, int by1) {
+  using M = LaneMap<SSN>;
+  const int x0 = max(bx0 - w.rx0, 0), x1 = min(bx1 - w.rx0, M::kW - 1);
+  const int y0 = max(by0 - w.ry0, 0), y1 = min(by1 - w.ry0, M::kH - 1);
+  uint32_t m = 0;
+#pragma unroll
+  for (int y = 0; y < M::kH; ++y)
+    if (y >= y0 && y <= y1 && x0 <= x1) m |= ((2u << x1) - (1u << x0)) << (y * M::kW);
+  uint32_t all = m;
+#pragma unroll
+  for (int i = 1; i < SSN; ++i) all |= m << (i * M::kPix);
+  return all;
+}
+
+// Stages ring entries head .. head + nh - 1 in rec, one lane per hit, and finds
+// the pixels each covers, 32 sign tests a lane (with several samples a lane,
+// or a large triangle: the pixels it may cover), for `hit`. Returns the number
+// of the hit's first pixel, and the number of pixels of all hits. `lanes`: the
+// owner lanes whose pixel exists. Normals: the records' normals and colours
+// are wanted too.
+template <int S, int SSN, bool Normals>
+__device__ __forceinline__ int stage_hits(const WarpTile& w, const TriSetup* __restrict__ setup, const uint32_t* ring,
+                                          TriSetup* rec, uint2* hit, uint32_t lanes, uint32_t head, int nh,
+                                          int& total) {
+  using M = LaneMap<SSN>;
+  constexpr bool kCentre = S == 1 && SSN == 1;
+  const uint32_t lt = (1u << w.lane) - 1u;
+  uint32_t cover = 0, info = 0;
+  if (w.lane < nh) {
+    const TriSetup* src = setup + ring[(head + w.lane) % kRing];
+    TriSetup& dst = rec[w.lane];
+    cp_async16(&dst.zc, &src->zc);
+    if (Normals) {
+      cp_async16(&dst.n0, &src->n0);
+      cp_async16(&dst.n1, &src->n1);
+      cp_async16(&dst.n2, &src->n2);
+    }
+    const int4 a = __ldg(&src->xy01), b = __ldg(&src->xy2f);
+    const int X0 = a.x, Y0 = a.y, X1 = a.z, Y1 = a.w, X2 = b.x, Y2 = b.y;
+    const uint32_t flags = (uint32_t)b.z;
+    info = ((uint32_t)w.lane << 11) | ((flags << 8) & 0xFF0000u);
+    if (flags & kFlagSmall) {
+      const int t0 = (int)(flags & 1u), t1 = (int)((flags >> 1) & 1u), t2 = (int)((flags >> 2) & 1u);
+      const int A0 = (Y1 - Y2) * 512, B0 = (X2 - X1) * 512, A1 = (Y2 - Y0) * 512, B1 = (X0 - X2) * 512;
+      const int ox = w.rx0 * 256 + (kCentre ? 128 : 0), oy = w.ry0 * 256 + (kCentre ? 128 : 0);
+      const int E0 = 2 * ((X2 - X1) * (oy - Y1) + (Y1 - Y2) * (ox - X1)) + t0 - 1;
+      const int E1 = 2 * ((X0 - X2) * (oy - Y2) + (Y2 - Y0) * (ox - X2)) + t1 - 1;
+      const int sum = 2 * ((X1 - X0) * (Y2 - Y0) - (Y1 - Y0) * (X2 - X0)) + t0 + t1 + t2 - 3;
+      dst.xy01 = make_int4(E0, E1, sum, b.w);
+      dst.xy2f = make_int4(A0, B0, A1, B1);
+      // from the last lane to the first, so that each sign shifts in below the ones before it
+      uint32_t out = 0;
+      if (S == 1) {
+#pragma unroll
+        for (int smp = SSN - 1; smp >= 0; --smp) {
+          int s0 = E0, s1 = E1;
+          if (!kCentre) {
+            const int2 sp = sample_pos<SSN>(smp);
+            s0 += (A0 >> 8) * sp.x + (B0 >> 8) * sp.y;
+            s1 += (A1 >> 8) * sp.x + (B1 >> 8) * sp.y;
+          }
+#pragma unroll
+          for (int y = M::kH - 1; y >= 0; --y)
+#pragma unroll
+            for (int x = M::kW - 1; x >= 0; --x) {
+              const int e0 = s0 + A0 * x + B0 * y, e1 = s1 + A1 * x + B1 * y;
+              out = __funnelshift_l((uint32_t)(e0 | e1 | (sum - e0 - e1)), out, 1);
+            }
+        }
+      } else {
+        // the largest value over the pixel's samples (all of them within 16 .. 240)
+        const int A2 = -(A0 + A1), B2 = -(B0 + B1);
+        auto most = [](int A, int B) {
+          return (max(A, 0) >> 8) * 240 + (min(A, 0) >> 8) * 16 + (max(B, 0) >> 8) * 240 + (min(B, 0) >> 8) * 16;
+        };
+        const int s0 = E0 + most(A0, B0), s1 = E1 + most(A1, B1), s2 = sum - E0 - E1 + most(A2, B2);
+#pragma unroll
+        for (int y = M::kH - 1; y >= 0; --y)
+#pragma unroll
+          for (int x = M::kW - 1; x >= 0; --x) {
+            const int e0 = s0 + A0 * x + B0 * y, e1 = s1 + A1 * x + B1 * y, e2 = s2 + A2 * x + B2 * y;
+            out = __funnelshift_l((uint32_t)(e0 | e1 | e2), out, 1);
+          }
+      }
+      cover = ~out & lanes;
+    } else {
+      info |= 0x80000000u;
+      dst.xy01 = a;
+      dst.xy2f = b;
+      cover = bbox_lanes<SSN>(w, min(X0, min(X1, X2)) >> 8, min(Y0, min(Y1, Y2)) >> 8, max(X0, max(X1, X2)) >> 8,
+                         max(Y0, max(Y1, Y2)) >> 8) & lanes;
+    }
+  }
+  const int n = __popc(cover);
+  int incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (w.lane >= o) incl += y;
+  }
+  total = __shfl_sync(kFull, incl, 31);
+  const uint32_t some = __ballot_sync(kFull, n > 0);
+  if (n > 0) hit[__popc(some & lt)] = make_uint2(info | (uint32_t)(incl - n), cover);
+  cp_async_wait_all();
+  __syncwarp();
+  return n > 0 ? incl - n : 0x40000000;
 }
 
 // S: samples each lane evaluates (MSAA coverage); SSN: samples mapped to
@@ -777,20 +882,8 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
   const TriSetup* __restrict__ setup = reinterpret_cast<const TriSetup*>(p.setup);
   const TriPersp* __restrict__ persp = reinterpret_cast<const TriPersp*>(p.persp);
   const uint32_t lt = (1u << w.lane) - 1u;
-  // owner lanes whose pixel exists, and those of the pixels in a bbox
+  // owner lanes whose pixel exists
   const uint32_t lanes = __ballot_sync(kFull, w.valid);
-  auto bbox_lanes = [&](int bx0, int by0, int bx1, int by1) {
-    const int x0 = max(bx0 - w.rx0, 0), x1 = min(bx1 - w.rx0, M::kW - 1);
-    const int y0 = max(by0 - w.ry0, 0), y1 = min(by1 - w.ry0, M::kH - 1);
-    uint32_t m = 0;
-#pragma unroll
-    for (int y = 0; y < M::kH; ++y)
-      if (y >= y0 && y <= y1 && x0 <= x1) m |= ((2u << x1) - (1u << x0)) << (y * M::kW);
-    uint32_t all = m;
-#pragma unroll
-    for (int i = 1; i < SSN; ++i) all |= m << (i * M::kPix);
-    return all;
-  };
   uint32_t nfrag = 0;  // warp-uniform
   uint32_t got = 0;    // fragments delivered to this lane's pixel
   int qn = 0;          // warp-uniform: queued fragments
@@ -799,88 +892,8 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
   for (int pass = 0; pass < Pol::kPasses; ++pass) {
     const bool shading = Pol::kPasses == 1 || pass == Pol::kPasses - 1;
 
-    // Stages ring entries head .. head + nh - 1, one lane per hit, and finds
-    // the pixels each covers, 32 sign tests a lane (with several samples a
-    // lane, or a large triangle: the pixels it may cover). Returns the number
-    // of the hit's first pixel, and the number of pixels of all hits.
     auto stage = [&](uint32_t head, int nh, int& total) {
-      uint32_t cover = 0, info = 0;
-      if (w.lane < nh) {
-        const TriSetup* src = setup + st.ring[(head + w.lane) % kRing];
-        TriSetup& dst = st.rec[w.lane];
-        cp_async16(&dst.zc, &src->zc);
-        cp_async16(&dst.n0, &src->n0);
-        cp_async16(&dst.n1, &src->n1);
-        cp_async16(&dst.n2, &src->n2);
-        const int4 a = __ldg(&src->xy01), b = __ldg(&src->xy2f);
-        const int X0 = a.x, Y0 = a.y, X1 = a.z, Y1 = a.w, X2 = b.x, Y2 = b.y;
-        const uint32_t flags = (uint32_t)b.z;
-        info = ((uint32_t)w.lane << 11) | ((flags << 8) & 0xFF0000u);
-        if (flags & kFlagSmall) {
-          const int t0 = (int)(flags & 1u), t1 = (int)((flags >> 1) & 1u), t2 = (int)((flags >> 2) & 1u);
-          const int A0 = (Y1 - Y2) * 512, B0 = (X2 - X1) * 512, A1 = (Y2 - Y0) * 512, B1 = (X0 - X2) * 512;
-          const int ox = w.rx0 * 256 + (kCentre ? 128 : 0), oy = w.ry0 * 256 + (kCentre ? 128 : 0);
-          const int E0 = 2 * ((X2 - X1) * (oy - Y1) + (Y1 - Y2) * (ox - X1)) + t0 - 1;
-          const int E1 = 2 * ((X0 - X2) * (oy - Y2) + (Y2 - Y0) * (ox - X2)) + t1 - 1;
-          const int sum = 2 * ((X1 - X0) * (Y2 - Y0) - (Y1 - Y0) * (X2 - X0)) + t0 + t1 + t2 - 3;
-          dst.xy01 = make_int4(E0, E1, sum, b.w);
-          dst.xy2f = make_int4(A0, B0, A1, B1);
-          // from the last lane to the first, so that each sign shifts in below the ones before it
-          uint32_t out = 0;
-          if (S == 1) {
-#pragma unroll
-            for (int smp = SSN - 1; smp >= 0; --smp) {
-              int s0 = E0, s1 = E1;
-              if (!kCentre) {
-                const int2 sp = sample_pos<SSN>(smp);
-                s0 += (A0 >> 8) * sp.x + (B0 >> 8) * sp.y;
-                s1 += (A1 >> 8) * sp.x + (B1 >> 8) * sp.y;
-              }
-#pragma unroll
-              for (int y = M::kH - 1; y >= 0; --y)
-#pragma unroll
-                for (int x = M::kW - 1; x >= 0; --x) {
-                  const int e0 = s0 + A0 * x + B0 * y, e1 = s1 + A1 * x + B1 * y;
-                  out = __funnelshift_l((uint32_t)(e0 | e1 | (sum - e0 - e1)), out, 1);
-                }
-            }
-          } else {
-            // the largest value over the pixel's samples (all of them within 16 .. 240)
-            const int A2 = -(A0 + A1), B2 = -(B0 + B1);
-            auto most = [](int A, int B) {
-              return (max(A, 0) >> 8) * 240 + (min(A, 0) >> 8) * 16 + (max(B, 0) >> 8) * 240 + (min(B, 0) >> 8) * 16;
-            };
-            const int s0 = E0 + most(A0, B0), s1 = E1 + most(A1, B1), s2 = sum - E0 - E1 + most(A2, B2);
-#pragma unroll
-            for (int y = M::kH - 1; y >= 0; --y)
-#pragma unroll
-              for (int x = M::kW - 1; x >= 0; --x) {
-                const int e0 = s0 + A0 * x + B0 * y, e1 = s1 + A1 * x + B1 * y, e2 = s2 + A2 * x + B2 * y;
-                out = __funnelshift_l((uint32_t)(e0 | e1 | e2), out, 1);
-              }
-          }
-          cover = ~out & lanes;
-        } else {
-          info |= 0x80000000u;
-          dst.xy01 = a;
-          dst.xy2f = b;
-          cover = bbox_lanes(min(X0, min(X1, X2)) >> 8, min(Y0, min(Y1, Y2)) >> 8, max(X0, max(X1, X2)) >> 8,
-                             max(Y0, max(Y1, Y2)) >> 8) & lanes;
-        }
-      }
-      const int n = __popc(cover);
-      int incl = n;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, incl, o);
-        if (w.lane >= o) incl += y;
-      }
-      total = __shfl_sync(kFull, incl, 31);
-      const uint32_t some = __ballot_sync(kFull, n > 0);
-      if (n > 0) st.hit[__popc(some & lt)] = make_uint2(info | (uint32_t)(incl - n), cover);
-      cp_async_wait_all();
-      __syncwarp();
-      return n > 0 ? incl - n : 0x40000000;
+      return stage_hits<S, SSN, true>(w, setup, st.ring, st.rec, st.hit, lanes, head, nh, total);
     };
 
     // Edge values of hit h, record T at owner lane `owner`'s shading point: its
@@ -1208,78 +1221,122 @@ __global__ void __launch_bounds__(32 * kRasterWarpsPerBlock,
 // ---------------------------------------------------------------------------
 // Opaque pass: opaque.frag.glsl:30-35, depth LESS with write (main.cpp:542-547).
 // ---------------------------------------------------------------------------
+// Per sample the nearest triangle, the first in primitive order among equal
+// depths, is kept in shared memory; each pixel is shaded at the end, once per
+// distinct triangle of its samples. Coverage as in the transparent pass.
+// Measured against every fragment shaded, hits tested one after the other by
+// all lanes, and targets cleared by fills beforehand: frames of Loop64
+// 1920x1080 with 40% opaque spheres 421 -> 353 us, Simple 1283x717 4x MSAA with
+// 30% 458 -> 382 us.
+// id: the triangle's place in primitive order, 2 t for triangle t or its first
+// half and 2 t + 1 for its second.
+template <int S>
+struct OpaqueStage {
+  TriSetup rec[kHits];  // (normals and colours unused)
+  uint2 hit[kHits];
+  uint32_t ring[kRing];
+  uint32_t z[S][32];
+  uint32_t id[S][32];
+};
+constexpr uint32_t kNoTriangle = 0xFFFFFFFFu;
+
+// Of the warp's fragments (pass: nearer than the sample's depth z), keeps per
+// sample the nearest, the lowest id among equal depths. Warp-uniform call.
+__device__ __forceinline__ void keep_nearest(uint32_t* z, uint32_t* id, bool pass, int owner, uint32_t zf,
+                                             uint32_t oid) {
+  if (!__any_sync(kFull, pass)) return;
+  if (pass) atomicMin(&z[owner], zf);
+  __syncwarp();
+  const bool win = pass && z[owner] == zf;  // (an earlier fragment of this depth would not have let it pass)
+  if (win) id[owner] = kNoTriangle;
+  __syncwarp();
+  if (win) atomicMin(&id[owner], oid);
+  __syncwarp();
+}
+
 template <int S>
 __device__ __forceinline__ void raster_opaque_body(const RasterParams& p, int cta) {
-  __shared__ TriSetup stage_all[kRasterWarpsPerBlock][kHits];
-  __shared__ uint2 bbox_all[kRasterWarpsPerBlock][kHits];
-  __shared__ uint32_t ring_all[kRasterWarpsPerBlock][kRing];
+  using M = LaneMap<1>;
+  __shared__ OpaqueStage<S> st_all[kRasterWarpsPerBlock];
   const int warp = threadIdx.x >> 5;
   const WarpTile w = warp_tile<1>(p, cta);
-  TriSetup* stage = stage_all[warp];
-  uint2* stage_bb = bbox_all[warp];
-  uint32_t* ring = ring_all[warp];
+  OpaqueStage<S>& st = st_all[warp];
   const TriSetup* __restrict__ setup = reinterpret_cast<const TriSetup*>(p.setup);
-  uint32_t dep[S];
-  float4 col[S];
+  const uint32_t lt = (1u << w.lane) - 1u;
+  const uint32_t lanes = __ballot_sync(kFull, w.valid);
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    dep[s] = w.valid ? p.depth[(size_t)s * p.P + w.pixel] : 0x3F800000u;
-    col[s] = w.valid ? p.opaque_color[(size_t)s * p.P + w.pixel] : p.background;
+    st.z[s][w.lane] = w.valid && !p.opaque_fresh ? p.depth[(size_t)s * p.P + w.pixel] : 0x3F800000u;
+    st.id[s][w.lane] = kNoTriangle;
   }
   const int tile = (int)((cta * kRasterWarpsPerBlock + warp) / oit::kWarpsPerTile) + p.tile_offset;
-  walk_pass<false>(p, w, ring, p.tile_begin[tile], p.tile_end[tile], [&](uint32_t head, int nh, bool) {
-    if (w.lane < nh) {
-      const uint32_t t = ring[(head + w.lane) % kRing];
-      const int4* src = reinterpret_cast<const int4*>(setup + t);
-      int4* dst = reinterpret_cast<int4*>(stage + w.lane);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) cp_async16(dst + k, src + k);
-      stage_bb[w.lane] = __ldg(&p.bbox[t]);
-    }
-    cp_async_wait_all();
-    __syncwarp();
+  walk_pass<false>(p, w, st.ring, p.tile_begin[tile], p.tile_end[tile], [&](uint32_t head, int nh, bool) {
+    int total = 0;
+    const int pre = stage_hits<S, 1, false>(w, setup, st.ring, st.rec, st.hit, lanes, head, nh, total);
+    int khi = -1;
 #pragma unroll 1
-    for (int k = 0; k < nh; ++k) {
-      if (!lane_in_bbox(stage_bb[k], w)) continue;  // no warp-collective operation follows
-      const TriSetup& T = stage[k];
-      const int4 a = T.xy01, b = T.xy2f;
-      const float4 zc = T.zc;
-      auto body = [&](auto etag) {
-        using E = decltype(etag);
-        const int bxp = w.px * 256, byp = w.py * 256;
-        uint32_t pass = 0;
-        uint32_t zs[S];
+    for (int base = 0; base < total; base += 32) {
+      const uint32_t rel = (uint32_t)(pre - base);
+      const uint32_t starts = __reduce_or_sync(kFull, rel < 32u ? 1u << rel : 0u);
+      const int j = khi + __popc(starts & (lt | (1u << w.lane)));
+      khi += __popc(starts);
+      const bool act = base + w.lane < total;
+      const uint2 h = st.hit[j];
+      const int k = (int)((h.x >> 11) & 31u);
+      const TriSetup& T = st.rec[k];
+      const int owner = act ? nth_bit(h.y, (uint32_t)(base + w.lane) - (h.x & 0x7FFu)) : w.lane;
+      const int dx = owner % M::kW, dy = owner / M::kW;
+      const uint32_t t = st.ring[(head + k) % kRing];
+      const uint32_t oid = t >= p.num_tris ? 2u * (t - p.num_tris) + 1u : 2u * t;
+      uint32_t zs[S];
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-          const int2 sp = sample_pos<S>(s);
-          const EdgesT<E> e = edges_at<E>(a, b, bxp + sp.x, byp + sp.y);
-          zs[s] = 0u;
-          if (inside(e, b.z)) {
-            const uint32_t z = __float_as_uint(depth_at(zc, e));
-            zs[s] = z;
-            if (z < dep[s]) pass |= 1u << s;
+      for (int s = 0; s < S; ++s) zs[s] = 0xFFFFFFFFu;
+      if (act) {
+        const int4 a = T.xy01, b = T.xy2f;
+        const float4 zc = T.zc;
+        if (!(h.x >> 31)) {
+          const int E0 = a.x + b.x * dx + b.y * dy, E1 = a.y + b.z * dx + b.w * dy;
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            const int2 sp = S > 1 ? sample_pos<S>(s) : make_int2(0, 0);  // (1x: taken at the centre)
+            const int e0 = E0 + (b.x >> 8) * sp.x + (b.y >> 8) * sp.y;
+            const int e1 = E1 + (b.z >> 8) * sp.x + (b.w >> 8) * sp.y;
+            const int e2 = a.z - e0 - e1;
+            if ((e0 | e1 | e2) >= 0)
+              zs[s] = __float_as_uint(depth_from(zc, to_float((e1 + 1) >> 1), to_float((e2 + 1) >> 1)));
+          }
+        } else {
+          const int bxp = (w.rx0 + dx) * 256, byp = (w.ry0 + dy) * 256;
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            const int2 sp = sample_pos<S>(s);
+            const Edges e = edges_at<long long>(a, b, bxp + sp.x, byp + sp.y);
+            if (inside(e, b.z)) zs[s] = __float_as_uint(depth_at(zc, e));
           }
         }
-        if (!pass) return;
-        const EdgesT<E> ec = edges_at<E>(a, b, bxp + 128, byp + 128);
-        const Shade sh = shade(T, ec, nullptr);
-        const float4 c = make_float4(sh.r, sh.g, sh.b, 1.0f);
+      }
 #pragma unroll
-        for (int s = 0; s < S; ++s)
-          if (pass & (1u << s)) {
-            dep[s] = zs[s];
-            col[s] = c;
-          }
-      };
-      if (b.z & kFlagSmall) body(int(0)); else body((long long)0);
+      for (int s = 0; s < S; ++s) keep_nearest(st.z[s], st.id[s], zs[s] < st.z[s][owner], owner, zs[s], oid);
     }
   });
-  if (w.valid) {
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      p.depth[(size_t)s * p.P + w.pixel] = dep[s];
-      p.opaque_color[(size_t)s * p.P + w.pixel] = col[s];
+  if (!w.valid) return;
+  uint32_t shaded = kNoTriangle;
+  float4 c = p.background;
+#pragma unroll 1
+  for (int s = 0; s < S; ++s) {
+    const uint32_t id = st.id[s][w.lane];
+    if (id == kNoTriangle && !p.opaque_fresh) continue;
+    if (id != shaded) {
+      c = p.background;
+      if (id != kNoTriangle) {
+        const TriSetup& T = setup[(id & 1u) ? p.num_tris + (id >> 1) : id >> 1];
+        const Shade sh = shade(T, edges_at<long long>(T.xy01, T.xy2f, w.px * 256 + 128, w.py * 256 + 128), nullptr);
+        c = make_float4(sh.r, sh.g, sh.b, 1.0f);
+      }
+      shaded = id;
     }
+    p.depth[(size_t)s * p.P + w.pixel] = st.z[s][w.lane];
+    p.opaque_color[(size_t)s * p.P + w.pixel] = c;
   }
 }
 
