@@ -111,12 +111,13 @@ struct oit_context {
 
   DevBuf depth, opaque_color, color, abuf, aux, auxdepth, counter, accum, reveal, out, out_linear, err, frag;
   DevBuf bbox, setup, persp, pair_count, pair_offset, scan_tmp, total;
-  DevBuf keys, tris, keys_alt, tris_alt, hist, tile_begin, tile_end;
+  DevBuf keys, tris, keys_alt, tris_alt, hist, tile_begin, tile_end, tile_order;
   DevBuf mesh_v, mesh_i;
   DevBuf scene_dev;  // proj_view then view, read by k_setup
   DevBuf lens;  // per 8x4 micro-tile fragment counts for the batched resolve
   size_t tri_cap = 0, pair_cap = 0;
   uint32_t bin_tris = 0, bin_opaque_from = 0;  // the last binned draw: triangles, first opaque one
+  bool bin_ordered = false;                    // its tiles are in order of list length
   bool opaque_valid = false;
   bool opaque_started = false;  // the frame's opaque targets are written (else its first opaque pass clears them)
   bool color_valid = false;
@@ -191,7 +192,7 @@ struct oit_context {
     if (scene_ring) cudaFreeHost(scene_ring);
     DevBuf* all[] = {&depth, &opaque_color, &color, &abuf, &aux, &auxdepth, &counter, &accum, &reveal, &out,
                      &out_linear, &err, &frag, &bbox, &setup, &persp, &pair_count, &pair_offset, &scan_tmp, &total,
-                     &keys, &tris, &keys_alt, &tris_alt, &hist, &tile_begin, &tile_end, &mesh_v, &mesh_i,
+                     &keys, &tris, &keys_alt, &tris_alt, &hist, &tile_begin, &tile_end, &tile_order, &mesh_v, &mesh_i,
                      &scene_dev, &lens};
     for (DevBuf* b : all) b->release();
   }
@@ -206,6 +207,11 @@ struct oit_context {
     return (alg() == oit::Alg::LinkedList || alg() == oit::Alg::Loop64) && st.record_format == OIT_RECORD_RGBA8 &&
            S == 1 && ssn == 1 && supersample == 1 && !(st.flags & OIT_FLAG_LINEAR_OUTPUT);
   }
+  // Tiles of a frame up to which its rasters take them by list length (the
+  // largest such frame measured, 3645 tiles, is 10% faster; one of 8160 2%
+  // slower); the views of a batch fill the GPU together and keep tile order.
+  static constexpr int kOrderMaxTiles = 4096;
+  size_t order_words() const { return (size_t)2 * oit::kOrderBuckets * (size_t)num_tiles; }
   int lens_stride() const { return (RW + 7) / 8; }
   int lens_rows() const { return (RH + 3) / 4; }
   size_t lens_count() const { return (size_t)lens_stride() * (size_t)lens_rows(); }
@@ -251,6 +257,8 @@ struct oit_context {
     OIT_TRY_CUDA(frag.ensure(8), "alloc frag");
     OIT_TRY_CUDA(tile_begin.ensure((size_t)2 * num_tiles * 4), "alloc bins");
     OIT_TRY_CUDA(tile_end.ensure((size_t)2 * num_tiles * 4), "alloc bins");
+    if (num_tiles <= kOrderMaxTiles)
+      OIT_TRY_CUDA(tile_order.ensure(order_words() * 4 + 2 * oit::kOrderBuckets * 4), "alloc order");
     OIT_TRY_CUDA(total.ensure(4), "alloc total");
     OIT_TRY_CUDA(scene_dev.ensure(kSceneBytes), "alloc scene");
     OIT_TRY_CUDA(cudaMallocHost(&scene_ring, kSceneSlots * kSceneBytes), "alloc pinned scene");
@@ -365,6 +373,10 @@ struct oit_context {
     b.scan_tmp = scan_tmp.as<uint32_t>();
     b.hist = hist.as<uint32_t>();
     b.total = total.as<uint32_t>();
+    if (tile_order.p && !in_batch) {
+      b.order = tile_order.as<uint32_t>();
+      b.order_count = b.order + order_words();
+    }
     b.capacity = pair_cap;
     // measured: the 64-view batch 18.64 ms at 8M against 18.96 at 1M; a
     // 2560x1440 MSAA-8 frame alone 6.38 ms at 1M against 6.51 at 8M
@@ -421,6 +433,7 @@ struct oit_context {
     bin_tris = count;
     bin_opaque_from = opaque_from;
     oit::Bins b = bins();
+    bin_ordered = b.order != nullptr;
     OIT_TRY_CUDA(oit::bin_setup_scan(sp, b, s, &launches), "bin_setup_scan");
     if (!ps) {
       if (capturing) return OIT_ERR_STATE;  // a captured frame never sizes bins
@@ -470,6 +483,11 @@ struct oit_context {
     p.tile_begin = tile_begin.as<uint32_t>();
     p.tile_end = tile_end.as<uint32_t>();
     p.tile_offset = tile_offset;
+    if (bin_ordered) {
+      const int kind = tile_offset != 0 ? 1 : 0;
+      p.tile_order = tile_order.as<uint32_t>() + (size_t)kind * oit::kOrderBuckets * (size_t)num_tiles;
+      p.order_count = tile_order.as<uint32_t>() + order_words() + kind * oit::kOrderBuckets;
+    }
     p.pair_total = total.as<uint32_t>();
     p.pair_offset = pair_offset.as<uint32_t>();
     p.pair_count = pair_count.as<uint32_t>();

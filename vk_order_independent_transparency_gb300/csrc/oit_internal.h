@@ -15,6 +15,7 @@ constexpr int kRasterWarpsPerBlock = 2;  // micro-tile warps per tile-raster CTA
 constexpr int kMaskShift = 24;
 constexpr uint32_t kTileKeyMask = (1u << kMaskShift) - 1u;
 constexpr uint32_t kEmpty32 = 0xFFFFFFFFu;
+constexpr int kOrderBuckets = 8;     // buckets of the tiles by list length
 
 struct Mat4 {
   float m[16];
@@ -70,6 +71,10 @@ struct Bins {
   uint32_t* scan_tmp;     // pair counts per 512-triangle block, scanned in place, then the scan's scratch
   uint32_t* hist;         // the radix sort's digit counts per chunk (and the scanned sort's scratch)
   uint32_t* total;        // [1] number of pairs (device)
+  // tiles of each kind by list length, [2][kOrderBuckets][num_tiles], and how
+  // many each bucket holds; null: not wanted
+  uint32_t* order;
+  uint32_t* order_count;
   size_t capacity;
   // the radix sort keeps a view's pairs in at most 128 chunks up to this many
   // pairs (a view sorted beside others: they fill the GPU), and beyond it
@@ -101,6 +106,10 @@ struct RasterParams {
   const uint32_t* tile_begin;    // indexed by tile + tile_offset
   const uint32_t* tile_end;
   int tile_offset;               // 0: opaque lists, num_tiles: transparent lists
+  // the pass's tiles by list length, [kOrderBuckets][tiles], and the buckets'
+  // counts; null: in tile order
+  const uint32_t* tile_order;
+  const uint32_t* order_count;
   const uint32_t* tile_tris;
   // the sorted pair keys beside tile_tris: tile id (bits 0-23) and the 8x4
   // micro-tiles of the tile that the triangle's bbox overlaps (bit 24 + k for

@@ -511,6 +511,7 @@ struct WeightedPolicy {
 // 8 * SSN warps cover the tile.
 struct WarpTile {
   int lane, px, py, rx0, ry0, rx1, ry1;
+  int tile;
   int mt;      // the 8x4 micro-tile of the tile that holds the warp's pixels
   int sample;  // the lane's sample with sample shading, else 0
   bool valid;
@@ -526,6 +527,33 @@ struct LaneMap {
   __device__ static int sample(int lane) { return lane / kPix; }
 };
 
+// The pass's tile number q: q itself, or with the tiles in buckets by list
+// length, taken in turn from the longest and from the shortest lists. A small
+// frame is resident as a whole but for its last tiles, and then waits for the
+// tile with the longest list; between them the short lists' tiles write their
+// (empty) A-buffers, which all at the end would be bound by memory. Measured in
+// tile order, longest first, in turn: Simple 1283x717 4x MSAA 382 / 344 / 346
+// us, Spinlock 800x512 253 / 236 / 242, linked list 1280x720 251 / 244 / 237,
+// Loop32 1001x563 4x sample shading 362 / 378 / 363; but WBOIT 3840x2160 3.25 /
+// 3.25 / 3.37 ms and Loop64 1920x1080 346 / 360 / 354 us: neighbouring tiles
+// read the same records, so larger frames keep the tile order. Warp-uniform.
+__device__ __forceinline__ int ordered_tile(const RasterParams& p, int q, int lane) {
+  if (!p.tile_order) return q;
+  constexpr int B = oit::kOrderBuckets;
+  q = (q & 1) ? p.tiles_x * p.tiles_y - 1 - (q >> 1) : q >> 1;
+  const int bucket = B - 1 - lane;  // lane 0: the longest lists
+  const uint32_t c = lane < B ? __ldg(&p.order_count[bucket]) : 0u;
+  uint32_t incl = c;
+#pragma unroll
+  for (int o = 1; o < B; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int at = __ffs((int)__ballot_sync(kFull, lane < B && (uint32_t)q < incl)) - 1;
+  const uint32_t before = __shfl_sync(kFull, incl - c, at);
+  return (int)__ldg(&p.tile_order[(size_t)(B - 1 - at) * (size_t)(p.tiles_x * p.tiles_y) + ((uint32_t)q - before)]);
+}
+
 // cta: the CTA's index within its view's grid.
 template <int SSN>
 __device__ __forceinline__ WarpTile warp_tile(const RasterParams& p, int cta) {
@@ -534,10 +562,11 @@ __device__ __forceinline__ WarpTile warp_tile(const RasterParams& p, int cta) {
   const int warp = threadIdx.x >> 5;
   w.lane = threadIdx.x & 31;
   const int gw = cta * (int)(blockDim.x >> 5) + warp;   // warp within the pass
-  const int tile = gw / (oit::kWarpsPerTile * SSN);
+  const int tile = ordered_tile(p, gw / (oit::kWarpsPerTile * SSN), w.lane);
   const int part = gw % (oit::kWarpsPerTile * SSN);     // the warp's part of the tile
   const int tx = tile % p.tiles_x, ty = tile / p.tiles_x;
   const int lx = (part % (16 / M::kW)) * M::kW, ly = (part / (16 / M::kW)) * M::kH;
+  w.tile = tile;
   w.mt = 2 * (ly >> 2) + (lx >> 3);
   w.rx0 = tx * 16 + lx;
   w.ry0 = ty * 16 + ly;
@@ -567,12 +596,14 @@ __device__ __forceinline__ bool bbox_hits(uint2 bb, const WarpTile& w) {
   return !(bx1 < w.rx0 || bx0 > w.rx1 || by1 < w.ry0 || by0 > w.ry1);
 }
 
-// Hits a warp processes at once, and the ring its list walk collects them in
-// (at most 31 left over and 32 new ones).
+// Hits a warp processes at once, the list entries its walk tests at a time,
+// and the ring it collects hits in (at most kHits - 1 left over and kScan new
+// ones).
 constexpr int kHits = 32;
-constexpr int kRing = 64;
+constexpr int kScan = 64;
+constexpr int kRing = 128;
 
-// Walks [beg, end) of the tile list in primitive order, 32 entries at a time,
+// Walks [beg, end) of the tile list in primitive order, kScan entries at a time,
 // and collects the triangles whose bbox touches the warp's pixels in `ring`;
 // chunk(head, nh, last) then processes ring entries head .. head + nh - 1
 // (modulo kRing), kHits of them until the list ends, and once more with nh = 0
@@ -592,36 +623,53 @@ __device__ __forceinline__ void walk_list(const RasterParams& p, const WarpTile&
   const uint32_t lt = (1u << w.lane) - 1u;
   const uint32_t mbit = 1u << (oit::kMaskShift + w.mt);
   const bool test = Fine || ident || limit != 0xFFFFFFFFu;
-  uint32_t key = 0, t = 0;  // the lane's entry of the block at pos, fetched ahead
-  auto fetch = [&](uint32_t i) {
-    key = 0;
-    if (i >= end) return;
-    if (ident) {
-      key = mbit;
-      t = (i & 1u) ? p.num_tris + (i >> 1) : (i >> 1);
-    } else {
-      key = __ldg(&p.tile_keys[i]);
-      t = __ldg(&p.tile_tris[i]);
+  // the lane's entries of the block at pos, fetched while the one before it is
+  // tested: a block's loads take an L2 round trip whatever its size
+  constexpr int kPer = kScan / 32;
+  uint32_t key[kPer], t[kPer];
+  auto fetch = [&](uint32_t pos) {
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const uint32_t i = pos + 32u * u + w.lane;
+      key[u] = 0;
+      if (i >= end) continue;
+      if (ident) {
+        key[u] = mbit;
+        t[u] = (i & 1u) ? p.num_tris + (i >> 1) : (i >> 1);
+      } else {
+        key[u] = __ldg(&p.tile_keys[i]);
+        t[u] = __ldg(&p.tile_tris[i]);
+      }
     }
   };
   uint32_t pos = beg, head = 0, cnt = 0;
-  fetch(pos + w.lane);
+  fetch(pos);
 #pragma unroll 1
   for (;;) {
 #pragma unroll 1
     while (cnt < kHits && pos < end) {
-      bool hit = (key & mbit) != 0u;
-      const uint32_t tc = t, i = pos + w.lane;
-      pos += 32;
-      fetch(pos + w.lane);
-      if (test && hit) {
-        if (ident && (i & 1u) && !(__ldg(&p.bbox[i >> 1]).y >> 31)) hit = false;
-        else if (Fine || ident) hit = bbox_hits(__ldg(&p.bbox[tc]), w);
-        if ((tc >= p.num_tris ? tc - p.num_tris : tc) >= limit) hit = false;
+      bool hit[kPer];
+      uint32_t tc[kPer];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        hit[u] = (key[u] & mbit) != 0u;
+        tc[u] = t[u];
       }
-      const uint32_t m = __ballot_sync(kFull, hit);
-      if (hit) ring[(head + cnt + __popc(m & lt)) % kRing] = tc;
-      cnt += __popc(m);
+      const uint32_t at = pos;
+      pos += kScan;
+      fetch(pos);
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        if (test && hit[u]) {
+          const uint32_t i = at + 32u * u + w.lane;
+          if (ident && (i & 1u) && !(__ldg(&p.bbox[i >> 1]).y >> 31)) hit[u] = false;
+          else if (Fine || ident) hit[u] = bbox_hits(__ldg(&p.bbox[tc[u]]), w);
+          if ((tc[u] >= p.num_tris ? tc[u] - p.num_tris : tc[u]) >= limit) hit[u] = false;
+        }
+        const uint32_t m = __ballot_sync(kFull, hit[u]);
+        if (hit[u]) ring[(head + cnt + __popc(m & lt)) % kRing] = tc[u];
+        cnt += __popc(m);
+      }
     }
     const int nh = (int)min(cnt, (uint32_t)kHits);
     __syncwarp();
@@ -676,19 +724,31 @@ __device__ __forceinline__ void walk_pass(const RasterParams& p, const WarpTile&
 //  hit   the hits that cover a pixel: number of the first covered one (bits
 //        0-10), record (bits 11-15), alpha code (bits 16-23), bit 31: not
 //        small; and the covered pixels, one bit per owner lane;
-//  ent   queued fragments: record (bits 0-4), owner lane (bits 8-12), coverage
-//        (bits 16-23); depth;
+//  ent   queued fragments: depth, and with several samples a lane the hit (bits
+//        0-4), owner lane (bits 8-12) and coverage (bits 16-23);
 //  mine  per 32 queued fragments and lane: the fragments of the lane's pixel;
 //  ring  triangles collected by the walk;
 //  then the policy's payload per queued fragment.
+template <bool Samples>
+struct QueueEntry {
+  uint32_t depth;
+};
+template <>
+struct QueueEntry<true> {
+  uint32_t depth, info;
+};
+template <bool Samples>
 struct WarpStage {
   TriSetup rec[kHits];
   uint2 hit[kHits];
-  uint2 ent[kQueue];
+  QueueEntry<Samples> ent[kQueue];
   uint32_t mine[kQueue / 32][32];
   uint32_t ring[kRing];
 };
-__host__ __device__ constexpr size_t warp_stage_bytes(int payload) { return sizeof(WarpStage) + (size_t)kQueue * payload; }
+template <int S>
+__host__ __device__ constexpr size_t warp_stage_bytes(int payload) {
+  return sizeof(WarpStage<(S > 1)>) + (size_t)kQueue * payload;
+}
 
 // Position of set bit n (0 = the lowest) of m; n < popc(m).
 __device__ __forceinline__ int nth_bit(uint32_t m, uint32_t n) {
@@ -858,12 +918,13 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
   const WarpTile w = warp_tile<SSN>(p, cta);
   const uint32_t elem = (uint32_t)w.sample * p.P + w.pixel;  // this lane's sample of the pixel
   const int payload = Pol::payload_bytes(p.tail, p.record_fp32);
-  unsigned char* wbase = smem_raw + (size_t)warp * warp_stage_bytes(payload);
-  WarpStage& st = *reinterpret_cast<WarpStage*>(wbase);
+  unsigned char* wbase = smem_raw + (size_t)warp * warp_stage_bytes<S>(payload);
+  using Stage = WarpStage<(S > 1)>;
+  Stage& st = *reinterpret_cast<Stage*>(wbase);
   FragPay pay;
-  pay.rgba = reinterpret_cast<float4*>(wbase + sizeof(WarpStage));
-  pay.packed = reinterpret_cast<uint32_t*>(wbase + sizeof(WarpStage) + (payload >= 16 ? kQueue * 16 : 0));
-  unsigned char* pol_smem = smem_raw + (size_t)(blockDim.x >> 5) * warp_stage_bytes(payload) +
+  pay.rgba = reinterpret_cast<float4*>(wbase + sizeof(Stage));
+  pay.packed = reinterpret_cast<uint32_t*>(wbase + sizeof(Stage) + (payload >= 16 ? kQueue * 16 : 0));
+  unsigned char* pol_smem = smem_raw + (size_t)(blockDim.x >> 5) * warp_stage_bytes<S>(payload) +
                             (size_t)warp * Pol::smem_bytes_per_warp(p.L, p.coverage, p.record_fp32);
 
   PixelTargets<S> tg;
@@ -877,7 +938,7 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
 #pragma unroll
   for (int i = 0; i < kQueue / 32; ++i) st.mine[i][w.lane] = 0u;
 
-  const int tile = (int)((cta * (blockDim.x >> 5) + warp) / (oit::kWarpsPerTile * SSN)) + p.tile_offset;
+  const int tile = w.tile + p.tile_offset;
   const uint32_t beg = p.tile_begin[tile], end = p.tile_end[tile];
   const TriSetup* __restrict__ setup = reinterpret_cast<const TriSetup*>(p.setup);
   const TriPersp* __restrict__ persp = reinterpret_cast<const TriPersp*>(p.persp);
@@ -1001,10 +1062,11 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
       while (m) {
         const int j = __ffsll((long long)m) - 1;
         m &= m - 1;
-        const uint2 e = st.ent[j];
+        const auto e = st.ent[j];
         Frag f;
-        f.depth = e.y;
-        f.cover = S > 1 ? e.x >> 16 : 1u;
+        f.depth = e.depth;
+        f.cover = 1u;
+        if constexpr (S > 1) f.cover = e.info >> 16;
         f.packed = shading ? pay.packed[j] : 0u;
         if constexpr (!Pol::kDirect) pol.fragment(p, pass, f, pay, j, tg);
       }
@@ -1054,7 +1116,7 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
               } else {
                 if (pass_z) {
                   const int e = qn + __popc(pm & lt);
-                  st.ent[e] = make_uint2(0u, f.depth);
+                  st.ent[e].depth = f.depth;
                   atomicOr(&st.mine[e >> 5][owner], 1u << (e & 31));
                   if (shading) {
                     shade_fragment(h, head, T, v, f, sh);
@@ -1106,7 +1168,7 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
             const uint32_t m = __ballot_sync(kFull, cover != 0);
             if (cover) {
               const int e = qn + __popc(m & lt);
-              st.ent[e] = make_uint2((uint32_t)j | ((uint32_t)owner << 8) | (cover << 16), __float_as_uint(zcen));
+              st.ent[e] = {__float_as_uint(zcen), (uint32_t)j | ((uint32_t)owner << 8) | (cover << 16)};
               if (!Pol::kDirect) atomicOr(&st.mine[e >> 5][owner], 1u << (e & 31));
             }
             qn += __popc(m);
@@ -1121,9 +1183,9 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
           while (shading && qn > qs && (done || qn > kQueue - 32 || (Pol::kDirect && qn >= 32))) {
             const int e = qs + w.lane;
             const bool act = e < qn;
-            const uint2 en = st.ent[e % kQueue];
-            const int owner = (int)((en.x >> 8) & 31u);
-            const uint2 h = st.hit[en.x & 31u];
+            const auto en = st.ent[e % kQueue];
+            const int owner = (int)((en.info >> 8) & 31u);
+            const uint2 h = st.hit[en.info & 31u];
             const TriSetup& T = st.rec[(h.x >> 11) & 31u];
             const int cnt = min(qn - qs, 32);
             uint32_t node0 = 0;
@@ -1133,14 +1195,14 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
             float alpha = 0.f;
             if (act) {
               float3 v;
-              f.cover = (en.x >> 16) & 255u;
-              f.depth = en.y;
+              f.cover = (en.info >> 16) & 255u;
+              f.depth = en.depth;
               edges(h, T, owner, v, alpha);
               shade_fragment(h, head, T, v, f, sh);
             }
             if constexpr (Pol::kDirect) {
               write_direct(act, cnt == 32 ? kFull : (1u << cnt) - 1u, owner, f, sh, alpha, node0);
-              const uint2 nx = st.ent[32 + w.lane];
+              const auto nx = st.ent[32 + w.lane];
               __syncwarp();
               st.ent[w.lane] = nx;
               qn -= cnt;
@@ -1269,7 +1331,7 @@ __device__ __forceinline__ void raster_opaque_body(const RasterParams& p, int ct
     st.z[s][w.lane] = w.valid && !p.opaque_fresh ? p.depth[(size_t)s * p.P + w.pixel] : 0x3F800000u;
     st.id[s][w.lane] = kNoTriangle;
   }
-  const int tile = (int)((cta * kRasterWarpsPerBlock + warp) / oit::kWarpsPerTile) + p.tile_offset;
+  const int tile = w.tile + p.tile_offset;
   walk_pass<false>(p, w, st.ring, p.tile_begin[tile], p.tile_end[tile], [&](uint32_t head, int nh, bool) {
     int total = 0;
     const int pre = stage_hits<S, 1, false>(w, setup, st.ring, st.rec, st.hit, lanes, head, nh, total);
@@ -1359,7 +1421,7 @@ namespace oitd {
 template <template <int> class Pol, int S, int SSN, int WPSM>
 cudaError_t launch_transparent_w(const RasterParams& p, cudaStream_t s) {
   const size_t smem = (size_t)kRasterWarpsPerBlock *
-                      (warp_stage_bytes(Pol<S>::payload_bytes(p.tail, p.record_fp32)) +
+                      (warp_stage_bytes<S>(Pol<S>::payload_bytes(p.tail, p.record_fp32)) +
                        Pol<S>::smem_bytes_per_warp(p.L, p.coverage, p.record_fp32));
   if (smem > 48 * 1024) {
     // raise the kernel's dynamic shared memory cap once per device (never
@@ -1397,7 +1459,7 @@ template <template <int> class Pol, int S, int SSN>
 cudaError_t launch_transparent_mv_s(const oit::MvRaster& mv, cudaStream_t s) {
   size_t per_warp = 0;
   for (int i = 0; i < mv.n; ++i)
-    per_warp = std::max(per_warp, warp_stage_bytes(Pol<S>::payload_bytes(mv.v[i].tail, mv.v[i].record_fp32)) +
+    per_warp = std::max(per_warp, warp_stage_bytes<S>(Pol<S>::payload_bytes(mv.v[i].tail, mv.v[i].record_fp32)) +
                                       Pol<S>::smem_bytes_per_warp(mv.v[i].L, mv.v[i].coverage, mv.v[i].record_fp32));
   const size_t smem = (size_t)kRasterWarpsPerBlock * per_warp;
   if (smem > 48 * 1024) {

@@ -17,8 +17,7 @@
 //                 chunks (digit counts, then a scatter with warp-private
 //                 ranks), so every tile's list keeps primitive order (the
 //                 mask bits ride along unsorted);
-//   k_tile_bounds begin/end of each tile's list (where the sorted tile id
-//                 changes).
+//   k_tile_lists  begin/end of each tile's list, and the tiles by list length.
 #include <algorithm>
 #include <cstdio>
 
@@ -494,8 +493,9 @@ __global__ void __launch_bounds__(kEmitTile) k_emit(const uint32_t* __restrict__
                                                     uint32_t opaque_from, uint32_t num_tiles,
                                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ tris,
                                                     size_t capacity, const uint32_t* __restrict__ total,
-                                                    uint32_t* err) {
+                                                    uint32_t* err, uint32_t* order_count) {
   __shared__ uint32_t smem[64];
+  if (order_count && blockIdx.x == 0 && threadIdx.x < 2 * kOrderBuckets) order_count[threadIdx.x] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && *total > capacity) atomicOr(err, 1u);  // OIT_DEVERR_BIN_OVERFLOW
   const uint32_t t = blockIdx.x * kEmitTile + threadIdx.x;
   const uint32_t c = t < n ? __ldg(&pair_count[t]) : 0u;
@@ -656,21 +656,53 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
   }
 }
 
-// [begin, end) of every tile's pair range in the sorted keys: every position
-// where the key changes ends the previous key's range and begins the next
-// one's. Both arrays start at zero, so tiles without pairs read an empty range.
-__global__ void __launch_bounds__(256) k_tile_bounds(const uint32_t* __restrict__ keys,
-                                                     const uint32_t* __restrict__ total, size_t capacity,
-                                                     uint32_t num_keys, uint32_t* __restrict__ begin,
-                                                     uint32_t* __restrict__ end) {
+// [begin, end) of every key's pair range in the sorted keys, one key a thread:
+// its first pair by binary search, its end from the next key's thread. A search
+// is ~20 loads deep, most of them shared by the block's threads; marking every
+// change of the sorted keys instead reads all pairs and needs both arrays
+// cleared.
+// With `order`, each kind's tiles are also put into kOrderBuckets buckets by
+// list length (a factor of two each), for the rasters to start with the longest
+// lists: order[(kind * kOrderBuckets + bucket) * num_tiles + ...], order_count[kind * kOrderBuckets + bucket].
+constexpr int kListKeys = 256;  // keys per block (of kListKeys + 32 threads)
+
+__global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* __restrict__ keys,
+                                                              const uint32_t* __restrict__ total, size_t capacity,
+                                                              uint32_t num_tiles, uint32_t* __restrict__ begin,
+                                                              uint32_t* __restrict__ end,
+                                                              uint32_t* __restrict__ order,
+                                                              uint32_t* __restrict__ order_count) {
+  __shared__ uint32_t first[kListKeys + 1];
+  __shared__ uint32_t cnt[2 * kOrderBuckets], base[2 * kOrderBuckets];
   const uint32_t n = (uint32_t)pair_count_of(total, capacity);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-    const uint32_t cur = i < n ? keys[i] & kTileKeyMask : num_keys;
-    const uint32_t prev = i > 0 ? keys[i - 1] & kTileKeyMask : 0xFFFFFFFFu;
-    if (cur == prev) continue;
-    if (i > 0 && prev < num_keys) end[prev] = i;
-    if (cur < num_keys) begin[cur] = i;
+  const uint32_t k = blockIdx.x * kListKeys + threadIdx.x;
+  if (threadIdx.x < 2 * kOrderBuckets) cnt[threadIdx.x] = 0;
+  if (threadIdx.x <= kListKeys) {
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if ((__ldg(&keys[mid]) & kTileKeyMask) < k) lo = mid + 1; else hi = mid;
+    }
+    first[threadIdx.x] = lo;
   }
+  __syncthreads();
+  const bool mine = threadIdx.x < kListKeys && k < 2u * num_tiles;
+  uint32_t slot = 0, rank = 0;
+  if (mine) {
+    const uint32_t lo = first[threadIdx.x], hi = first[threadIdx.x + 1];
+    begin[k] = lo;
+    end[k] = hi;
+    // bucket 0: fewer than 64 pairs, then a factor of two each
+    slot = (k < num_tiles ? 0u : (uint32_t)kOrderBuckets) +
+           min((uint32_t)max(26 - __clz((hi - lo) | 1u), 0), (uint32_t)kOrderBuckets - 1u);
+  }
+  if (!order) return;
+  if (mine) rank = atomicAdd(&cnt[slot], 1u);
+  __syncthreads();
+  if (threadIdx.x < 2 * kOrderBuckets && cnt[threadIdx.x])
+    base[threadIdx.x] = atomicAdd(&order_count[threadIdx.x], cnt[threadIdx.x]);
+  __syncthreads();
+  if (mine) order[(size_t)slot * num_tiles + base[slot] + rank] = k < num_tiles ? k : k - num_tiles;
 }
 
 __global__ void k_fill_u32(uint32_t* dst, uint32_t v, size_t n) {
@@ -771,9 +803,11 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
   if (n > 0) {
     k_emit<<<(unsigned)emit_blocks(n), kEmitTile, 0, s>>>(sp.pair_count, b.pair_offset, b.scan_tmp, sp.bbox, n,
                                                           sp.tiles_x, sp.opaque_from, (uint32_t)sp.num_tiles, b.keys,
-                                                          b.tris, b.capacity, b.total, error);
+                                                          b.tris, b.capacity, b.total, error, b.order_count);
     ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  } else if (b.order && (e = cudaMemsetAsync(b.order_count, 0, 2 * kOrderBuckets * 4, s)) != cudaSuccess) {
+    return e;  // (k_emit clears it otherwise)
   }
   const size_t chunk = sort_chunk(b.capacity, b.sort_direct_max);
   const uint32_t nchunks = (uint32_t)std::max<size_t>((b.capacity + chunk - 1) / chunk, 1);
@@ -797,13 +831,8 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
     std::swap(b.tris, b.tris_alt);
   }
   // ranges of both kinds: [0, num_tiles) opaque, [num_tiles, 2 num_tiles) transparent
-  const size_t range_bytes = (size_t)2 * num_tiles * sizeof(uint32_t);
-  if ((e = cudaMemsetAsync(b.tile_begin, 0, range_bytes, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(b.tile_end, 0, range_bytes, s)) != cudaSuccess) return e;
-  const size_t nb = std::min<size_t>((b.capacity + 256) / 256, 152 * 16);
-  k_tile_bounds<<<(unsigned)std::max<size_t>(nb, 1), 256, 0, s>>>(b.keys, b.total, b.capacity,
-                                                                  (uint32_t)(2 * num_tiles), b.tile_begin,
-                                                                  b.tile_end);
+  k_tile_lists<<<(unsigned)((2 * num_tiles + kListKeys - 1) / kListKeys), kListKeys + 32, 0, s>>>(
+      b.keys, b.total, b.capacity, (uint32_t)num_tiles, b.tile_begin, b.tile_end, b.order, b.order_count);
   ++*launches;
   return cudaGetLastError();
 }
