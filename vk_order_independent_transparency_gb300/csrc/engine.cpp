@@ -358,6 +358,10 @@ struct oit_context {
     sp.setup = setup.p;
     sp.persp = (alg() == oit::Alg::Weighted && opaque_from > 0) ? persp.p : nullptr;
     sp.pair_count = pair_count.as<uint32_t>();
+    if (clear_in_setup) {
+      sp.clear_fragments = frag.as<unsigned long long>();
+      if (alg() == oit::Alg::LinkedList) sp.clear_counter = counter.as<uint32_t>();
+    }
     return sp;
   }
 
@@ -386,8 +390,8 @@ struct oit_context {
 
   // Pair-count history per draw signature: the first draw of a signature reads
   // its pair count back synchronously to size the bins; later draws run without
-  // a host round trip, sized from earlier frames (their counts are copied back
-  // asynchronously into pinned memory and picked up when ready).
+  // a host round trip, sized from earlier frames (their counts are stored by the
+  // binning in pinned memory and picked up when ready).
   struct PairStat {
     uint64_t key = 0;
     uint32_t known = 0;
@@ -434,6 +438,7 @@ struct oit_context {
     bin_opaque_from = opaque_from;
     oit::Bins b = bins();
     bin_ordered = b.order != nullptr;
+    sp.clear_order = b.order_count;
     OIT_TRY_CUDA(oit::bin_setup_scan(sp, b, s, &launches), "bin_setup_scan");
     if (!ps) {
       if (capturing) return OIT_ERR_STATE;  // a captured frame never sizes bins
@@ -451,18 +456,17 @@ struct oit_context {
       if (r != OIT_OK) return r;
       b = bins();
     }
+    b.host_total = ps->host_total;
     OIT_TRY_CUDA(oit::bin_sort(sp, b, key_bits, num_tiles, err.as<uint32_t>(), s, &launches), "bin_sort");
     // bin_sort may have swapped the ping-pong buffers
     if (b.keys != keys.as<uint32_t>()) {
       std::swap(keys, keys_alt);
       std::swap(tris, tris_alt);
     }
-    if (!ps->pending || capturing) {
-      OIT_TRY_CUDA(cudaMemcpyAsync(ps->host_total, total.p, 4, cudaMemcpyDeviceToHost, s), "d2h");
-      if (!capturing) {
-        OIT_TRY_CUDA(cudaEventRecord(ps->ev, s), "event");
-        ps->pending = true;
-      }
+    // (the tile-list kernel stores the pair count in host_total)
+    if (!ps->pending && !capturing) {
+      OIT_TRY_CUDA(cudaEventRecord(ps->ev, s), "event");
+      ps->pending = true;
     }
     if (capturing) graph_stats.push_back(ps->key);
     return OIT_OK;
@@ -742,6 +746,7 @@ struct oit_context {
   // raster = false (a batch whose rasters run as multi-view launches): the
   // frame stops after binning; frame_has_opaque tells whether it has an opaque pass.
   bool frame_has_opaque = false;
+  bool clear_in_setup = false;  // the frame's setup kernel does clear_transparent's work
   int render_frame_body(const oit::MeshRef& mesh, uint32_t tpo, int32_t percent, uint8_t* out_dev, cudaStream_t s,
                         bool resolve = true, bool raster = true) {
     const uint32_t num_objects = mesh.num_triangles / tpo;
@@ -750,12 +755,14 @@ struct oit_context {
     const uint32_t num_opaque = num_objects - num_transparent;
     const uint32_t nt = num_transparent * tpo, total_tris = num_objects * tpo;
     int r = begin_frame(s);
-    if (r == OIT_OK) r = clear_transparent(s);
+    if (r == OIT_OK && total_tris == 0) r = clear_transparent(s);
     if (r == OIT_OK && num_opaque > 0) r = ensure_opaque_buffers();
     if (r != OIT_OK) return r;
     opaque_valid = num_opaque > 0;
     cudaEvent_t t0 = prof_begin(s);
+    clear_in_setup = true;
     r = bin(mesh, 0, total_tris, nt, s);
+    clear_in_setup = false;
     if (r != OIT_OK) return r;
     prof_end(OIT_PROF_TRANSPARENT_BIN, t0, s);
     frame_has_opaque = num_opaque > 0;

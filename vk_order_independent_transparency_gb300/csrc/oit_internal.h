@@ -47,6 +47,11 @@ struct SetupParams {
   void* setup;            // TriSetup records (96 B)
   void* persp;            // TriPersp records (32 B, WBOIT only) or null
   uint32_t* pair_count;   // [num_triangles] tiles overlapped by both halves (0 = culled)
+  // frame state the setup clears on the way (null: not): the fragment count,
+  // the linked list's node counter, the tile order's bucket counts
+  unsigned long long* clear_fragments;
+  uint32_t* clear_counter;
+  uint32_t* clear_order;
 };
 
 // The engine's view of a frame's geometry: a flattened triangle mesh
@@ -75,6 +80,7 @@ struct Bins {
   // many each bucket holds; null: not wanted
   uint32_t* order;
   uint32_t* order_count;
+  uint32_t* host_total;   // pinned host memory that receives the pair count; null: not wanted
   size_t capacity;
   // the radix sort keeps a view's pairs in at most 128 chunks up to this many
   // pairs (a view sorted beside others: they fill the GPU), and beyond it

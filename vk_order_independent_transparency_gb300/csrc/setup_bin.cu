@@ -244,6 +244,11 @@ constexpr uint32_t kClipPending = 0xFFFFFFFFu;
 // vertices in registers and free of the clip's extra state.
 __global__ void __launch_bounds__(256, 4) k_setup(SetupParams p, int S) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0) {
+    if (p.clear_fragments && threadIdx.x == 0) *p.clear_fragments = 0ull;
+    if (p.clear_counter && threadIdx.x == 0) *p.clear_counter = 0u;
+    if (p.clear_order && threadIdx.x < 2 * kOrderBuckets) p.clear_order[threadIdx.x] = 0u;
+  }
   if (t >= p.num_triangles) return;
   ClipVert cv[3];
   const float* c0 = clip_vertices(p, t, cv);
@@ -493,9 +498,8 @@ __global__ void __launch_bounds__(kEmitTile) k_emit(const uint32_t* __restrict__
                                                     uint32_t opaque_from, uint32_t num_tiles,
                                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ tris,
                                                     size_t capacity, const uint32_t* __restrict__ total,
-                                                    uint32_t* err, uint32_t* order_count) {
+                                                    uint32_t* err) {
   __shared__ uint32_t smem[64];
-  if (order_count && blockIdx.x == 0 && threadIdx.x < 2 * kOrderBuckets) order_count[threadIdx.x] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && *total > capacity) atomicOr(err, 1u);  // OIT_DEVERR_BIN_OVERFLOW
   const uint32_t t = blockIdx.x * kEmitTile + threadIdx.x;
   const uint32_t c = t < n ? __ldg(&pair_count[t]) : 0u;
@@ -671,11 +675,13 @@ __global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* _
                                                               uint32_t num_tiles, uint32_t* __restrict__ begin,
                                                               uint32_t* __restrict__ end,
                                                               uint32_t* __restrict__ order,
-                                                              uint32_t* __restrict__ order_count) {
+                                                              uint32_t* __restrict__ order_count,
+                                                              uint32_t* host_total) {
   __shared__ uint32_t first[kListKeys + 1];
   __shared__ uint32_t cnt[2 * kOrderBuckets], base[2 * kOrderBuckets];
   const uint32_t n = (uint32_t)pair_count_of(total, capacity);
   const uint32_t k = blockIdx.x * kListKeys + threadIdx.x;
+  if (host_total && blockIdx.x == 0 && threadIdx.x == 0) *host_total = *total;
   if (threadIdx.x < 2 * kOrderBuckets) cnt[threadIdx.x] = 0;
   if (threadIdx.x <= kListKeys) {
     uint32_t lo = 0, hi = n;
@@ -803,11 +809,11 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
   if (n > 0) {
     k_emit<<<(unsigned)emit_blocks(n), kEmitTile, 0, s>>>(sp.pair_count, b.pair_offset, b.scan_tmp, sp.bbox, n,
                                                           sp.tiles_x, sp.opaque_from, (uint32_t)sp.num_tiles, b.keys,
-                                                          b.tris, b.capacity, b.total, error, b.order_count);
+                                                          b.tris, b.capacity, b.total, error);
     ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   } else if (b.order && (e = cudaMemsetAsync(b.order_count, 0, 2 * kOrderBuckets * 4, s)) != cudaSuccess) {
-    return e;  // (k_emit clears it otherwise)
+    return e;  // (k_setup clears it otherwise)
   }
   const size_t chunk = sort_chunk(b.capacity, b.sort_direct_max);
   const uint32_t nchunks = (uint32_t)std::max<size_t>((b.capacity + chunk - 1) / chunk, 1);
@@ -832,7 +838,8 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
   }
   // ranges of both kinds: [0, num_tiles) opaque, [num_tiles, 2 num_tiles) transparent
   k_tile_lists<<<(unsigned)((2 * num_tiles + kListKeys - 1) / kListKeys), kListKeys + 32, 0, s>>>(
-      b.keys, b.total, b.capacity, (uint32_t)num_tiles, b.tile_begin, b.tile_end, b.order, b.order_count);
+      b.keys, b.total, b.capacity, (uint32_t)num_tiles, b.tile_begin, b.tile_end, b.order, b.order_count,
+      b.host_total);
   ++*launches;
   return cudaGetLastError();
 }
