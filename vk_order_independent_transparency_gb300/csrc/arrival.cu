@@ -20,6 +20,7 @@
 #include "../../include/oit_gb300.h"
 #include "oit_device.cuh"
 #include "oit_internal.h"
+#include "oit_launch.cuh"
 
 namespace oit {
 using namespace oitd;
@@ -61,6 +62,7 @@ __device__ __forceinline__ bool locked_tail_blend(const ArrivalParams& p, uint32
 }
 
 __global__ void __launch_bounds__(32 * kArrivalWarps, 4) k_arrival_ll(ArrivalParams p) {
+  frame_order();
   __shared__ unsigned long long pre_s[kArrivalWarps][32];  // exclusive prefix of the bbox areas
   __shared__ uint4 geo_s[kArrivalWarps][32];               // bbox x0, y0, width; triangle
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(32 * kArrivalWarps, 4) k_arrival_ll(ArrivalPar
 
 // The colour target before the pass: the opaque colour (or the background).
 __global__ void k_arrival_init(ArrivalParams p) {
+  frame_order();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.P; i += gridDim.x * blockDim.x) {
     const float4 c = p.has_opaque ? p.opaque_color[i] : p.background;
     store_color(p.color, p.color_half != 0, i, c);
@@ -195,7 +198,7 @@ __global__ void k_arrival_init(ArrivalParams p) {
 cudaError_t launch_arrival_ll(const ArrivalParams& p, cudaStream_t s, uint64_t* launches) {
   if (p.P) {
     const unsigned blocks = (unsigned)std::min<size_t>(((size_t)p.P + 255) / 256, 152 * 16);
-    k_arrival_init<<<blocks, 256, 0, s>>>(p);
+    launch_in_frame(k_arrival_init, blocks, 256, 0, s, p);
     ++*launches;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -203,7 +206,7 @@ cudaError_t launch_arrival_ll(const ArrivalParams& p, cudaStream_t s, uint64_t* 
   if (p.num_tris) {
     const size_t warps = (2 * (size_t)p.num_tris + 31) / 32;
     const unsigned blocks = (unsigned)std::min<size_t>((warps + kArrivalWarps - 1) / kArrivalWarps, 152 * 16);
-    k_arrival_ll<<<blocks, 32 * kArrivalWarps, 0, s>>>(p);
+    launch_in_frame(k_arrival_ll, blocks, 32 * kArrivalWarps, 0, s, p);
     ++*launches;
   }
   return cudaGetLastError();

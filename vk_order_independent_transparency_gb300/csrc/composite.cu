@@ -13,6 +13,7 @@
 #include "list_walk.cuh"
 #include "oit_device.cuh"
 #include "oit_internal.h"
+#include "oit_launch.cuh"
 
 namespace oit {
 using namespace oitd;
@@ -234,6 +235,7 @@ enum Kind { kRecords = 0, kList = 1, kLoop = 2, kLoop64 = 3, kListF32 = 4 };
 
 template <int K, int L>
 __global__ void __launch_bounds__(256) k_composite(CompositeParams p) {
+  frame_order();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (x >= p.W || y >= p.H) return;
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(256) k_composite(CompositeParams p) {
 // WBOIT composite: oitWeighted.frag.glsl:98-108 with blend
 // ONE_MINUS_SRC_ALPHA / SRC_ALPHA (main.cpp:578-588), per sample.
 __global__ void __launch_bounds__(256) k_composite_weighted(CompositeParams p) {
+  frame_order();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (x >= p.W || y >= p.H) return;
@@ -305,12 +308,12 @@ template <int K>
 cudaError_t launch_kind(const CompositeParams& p, cudaStream_t s) {
   const dim3 grid((p.W + 31) / 32, (p.H + 7) / 8), block(256);
   switch (p.L) {
-    case 1: k_composite<K, 1><<<grid, block, 0, s>>>(p); break;
-    case 2: k_composite<K, 2><<<grid, block, 0, s>>>(p); break;
-    case 4: k_composite<K, 4><<<grid, block, 0, s>>>(p); break;
-    case 8: k_composite<K, 8><<<grid, block, 0, s>>>(p); break;
-    case 16: k_composite<K, 16><<<grid, block, 0, s>>>(p); break;
-    case 32: k_composite<K, 32><<<grid, block, 0, s>>>(p); break;
+    case 1: launch_in_frame(k_composite<K, 1>, grid, block, 0, s, p); break;
+    case 2: launch_in_frame(k_composite<K, 2>, grid, block, 0, s, p); break;
+    case 4: launch_in_frame(k_composite<K, 4>, grid, block, 0, s, p); break;
+    case 8: launch_in_frame(k_composite<K, 8>, grid, block, 0, s, p); break;
+    case 16: launch_in_frame(k_composite<K, 16>, grid, block, 0, s, p); break;
+    case 32: launch_in_frame(k_composite<K, 32>, grid, block, 0, s, p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -325,9 +328,9 @@ cudaError_t launch_composite(Alg alg, const CompositeParams& p, cudaStream_t s) 
     case Alg::Spinlock:
     case Alg::Interlock: return launch_kind<kRecords>(p, s);
     case Alg::LinkedList: return p.record_fp32 ? launch_kind<kListF32>(p, s) : launch_kind<kList>(p, s);
-    case Alg::Loop: k_composite<kLoop, 1><<<grid, block, 0, s>>>(p); return cudaGetLastError();
-    case Alg::Loop64: k_composite<kLoop64, 1><<<grid, block, 0, s>>>(p); return cudaGetLastError();
-    case Alg::Weighted: k_composite_weighted<<<grid, block, 0, s>>>(p); return cudaGetLastError();
+    case Alg::Loop: launch_in_frame(k_composite<kLoop, 1>, grid, block, 0, s, p); return cudaGetLastError();
+    case Alg::Loop64: launch_in_frame(k_composite<kLoop64, 1>, grid, block, 0, s, p); return cudaGetLastError();
+    case Alg::Weighted: launch_in_frame(k_composite_weighted, grid, block, 0, s, p); return cudaGetLastError();
     default: return cudaErrorInvalidValue;
   }
 }

@@ -4,8 +4,9 @@
 // walks its tile's triangle list (primitive order, from the bins), collects the
 // triangles whose bbox touches the micro-tile (the hits) and processes them 32
 // at a time: one lane per hit prepares its edge equations and finds the pixels
-// it covers, one lane per covered pixel shades a fragment, and the pixel's owner lane runs the algorithm's fragment body (the COLOR/DEPTH shader
-// of the reference) on that pixel's state, so every pixel sees its fragments in
+// it covers, one lane per covered pixel shades a fragment, and the pixel's
+// owner lane runs the algorithm's fragment body (the COLOR/DEPTH shader of the
+// reference) on that pixel's state, so every pixel sees its fragments in
 // primitive order -- the order the reference's hardware blender guarantees for
 // tail blending and the order ordered interlock guarantees for its critical
 // section. Per-pixel k-buffers live in shared memory or registers; the
@@ -18,6 +19,7 @@
 #include <algorithm>
 
 #include "oit_device.cuh"
+#include "oit_launch.cuh"
 
 namespace oitd {
 
@@ -930,7 +932,8 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
   PixelTargets<S> tg;
 #pragma unroll
   for (int s = 0; s < S; ++s)
-    tg.col[s] = p.has_opaque && w.valid ? p.opaque_color[(size_t)(SSN > 1 ? w.sample : s) * p.P + w.pixel] : p.background;
+    tg.col[s] = p.has_opaque && w.valid ? p.opaque_color[(size_t)(SSN > 1 ? w.sample : s) * p.P + w.pixel]
+                                        : p.background;
   // this lane's opaque depth (1.0 without an opaque pass)
   const uint32_t depth = S == 1 && p.has_opaque && w.valid ? p.depth[elem] : 0x3F800000u;
   Pol pol;
@@ -1265,6 +1268,7 @@ __device__ __forceinline__ int mv_view(const oit::MvRaster& mv, uint32_t block, 
 template <template <int> class Policy, int S, int SSN, int WPSM = Policy<S>::kWarpsPerSM>
 __global__ void __launch_bounds__(32 * kRasterWarpsPerBlock, (S == 1 ? WPSM : 24) / kRasterWarpsPerBlock)
     k_raster_transparent(RasterParams p) {
+  frame_order();
   raster_transparent_body<Policy, S, SSN>(p, (int)blockIdx.x);
 }
 
@@ -1275,6 +1279,7 @@ template <template <int> class Policy, int S, int SSN>
 __global__ void __launch_bounds__(32 * kRasterWarpsPerBlock,
                                   (S == 1 ? Policy<S>::kWarpsPerSM : 24) / kRasterWarpsPerBlock)
     k_raster_transparent_mv(const __grid_constant__ oit::MvRaster mv) {
+  frame_order();
   int cta;
   const int v = mv_view(mv, blockIdx.x, cta);
   raster_transparent_body<Policy, S, SSN>(mv.v[v], cta);
@@ -1404,11 +1409,14 @@ __device__ __forceinline__ void raster_opaque_body(const RasterParams& p, int ct
 
 template <int S>
 __global__ void __launch_bounds__(32 * kRasterWarpsPerBlock) k_raster_opaque(RasterParams p) {
+  frame_order();
   raster_opaque_body<S>(p, (int)blockIdx.x);
 }
 
 template <int S>
-__global__ void __launch_bounds__(32 * kRasterWarpsPerBlock) k_raster_opaque_mv(const __grid_constant__ oit::MvRaster mv) {
+__global__ void __launch_bounds__(32 * kRasterWarpsPerBlock)
+    k_raster_opaque_mv(const __grid_constant__ oit::MvRaster mv) {
+  frame_order();
   int cta;
   const int v = mv_view(mv, blockIdx.x, cta);
   raster_opaque_body<S>(mv.v[v], cta);
@@ -1436,9 +1444,8 @@ cudaError_t launch_transparent_w(const RasterParams& p, cudaStream_t s) {
       if (dev >= 0 && dev < 64) cap_set[dev] = (int)smem;
     }
   }
-  k_raster_transparent<Pol, S, SSN, WPSM><<<(unsigned)(p.tiles_x * p.tiles_y * SSN *
-                                                       (oit::kWarpsPerTile / kRasterWarpsPerBlock)),
-                                            32 * kRasterWarpsPerBlock, smem, s>>>(p);
+  const unsigned ctas = (unsigned)(p.tiles_x * p.tiles_y * SSN * (oit::kWarpsPerTile / kRasterWarpsPerBlock));
+  launch_in_frame(k_raster_transparent<Pol, S, SSN, WPSM>, ctas, 32 * kRasterWarpsPerBlock, smem, s, p);
   return cudaGetLastError();
 }
 
@@ -1475,7 +1482,7 @@ cudaError_t launch_transparent_mv_s(const oit::MvRaster& mv, cudaStream_t s) {
   }
   const uint32_t ctas = mv.n > 0 ? mv.cta_end[mv.n - 1] : 0u;
   if (!ctas) return cudaSuccess;
-  k_raster_transparent_mv<Pol, S, SSN><<<ctas, 32 * kRasterWarpsPerBlock, smem, s>>>(mv);
+  launch_in_frame(k_raster_transparent_mv<Pol, S, SSN>, ctas, 32 * kRasterWarpsPerBlock, smem, s, mv);
   return cudaGetLastError();
 }
 
@@ -1504,9 +1511,9 @@ inline cudaError_t launch_opaque_mv(const oit::MvRaster& mv, cudaStream_t s) {
   if (!ctas) return cudaSuccess;
   constexpr int kThreads = 32 * kRasterWarpsPerBlock;
   switch (mv.v[0].S) {
-    case 1: k_raster_opaque_mv<1><<<ctas, kThreads, 0, s>>>(mv); break;
-    case 4: k_raster_opaque_mv<4><<<ctas, kThreads, 0, s>>>(mv); break;
-    case 8: k_raster_opaque_mv<8><<<ctas, kThreads, 0, s>>>(mv); break;
+    case 1: launch_in_frame(k_raster_opaque_mv<1>, ctas, kThreads, 0, s, mv); break;
+    case 4: launch_in_frame(k_raster_opaque_mv<4>, ctas, kThreads, 0, s, mv); break;
+    case 8: launch_in_frame(k_raster_opaque_mv<8>, ctas, kThreads, 0, s, mv); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -1533,9 +1540,9 @@ inline cudaError_t launch_opaque(const RasterParams& p, cudaStream_t s) {
   const unsigned grid = (unsigned)(p.tiles_x * p.tiles_y * (oit::kWarpsPerTile / kRasterWarpsPerBlock));
   constexpr int kThreads = 32 * kRasterWarpsPerBlock;
   switch (p.S) {
-    case 1: k_raster_opaque<1><<<grid, kThreads, 0, s>>>(p); break;
-    case 4: k_raster_opaque<4><<<grid, kThreads, 0, s>>>(p); break;
-    case 8: k_raster_opaque<8><<<grid, kThreads, 0, s>>>(p); break;
+    case 1: launch_in_frame(k_raster_opaque<1>, grid, kThreads, 0, s, p); break;
+    case 4: launch_in_frame(k_raster_opaque<4>, grid, kThreads, 0, s, p); break;
+    case 8: launch_in_frame(k_raster_opaque<8>, grid, kThreads, 0, s, p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -23,6 +23,7 @@
 
 #include "oit_device.cuh"
 #include "oit_internal.h"
+#include "oit_launch.cuh"
 
 namespace oit {
 using namespace oitd;
@@ -243,6 +244,7 @@ constexpr uint32_t kClipPending = 0xFFFFFFFFu;
 // crossing triangle is marked for k_setup_clip, which keeps this kernel's
 // vertices in registers and free of the clip's extra state.
 __global__ void __launch_bounds__(256, 4) k_setup(SetupParams p, int S) {
+  frame_order();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x == 0) {
     if (p.clear_fragments && threadIdx.x == 0) *p.clear_fragments = 0ull;
@@ -304,6 +306,7 @@ constexpr int kEmitTile = kClipThreads * kEmitItems;
 // with block_sums, the block's pair count (after clipping) is written there,
 // the first level of the pair-offset scan. pair_count is 16-byte aligned.
 __global__ void __launch_bounds__(kClipThreads) k_setup_clip(SetupParams p, int S, uint32_t* __restrict__ block_sums) {
+  frame_order();
   __shared__ uint32_t warp_sums[kClipThreads / 32];
   const uint32_t n = p.num_triangles;
   const uint32_t t0 = blockIdx.x * kEmitTile + threadIdx.x * kEmitItems;
@@ -366,6 +369,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const uint32_t* __restrict__ in, size_t n,
                                                             uint32_t* __restrict__ sums) {
+  frame_order();
   __shared__ uint32_t smem[64];
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t s = 0;
@@ -377,9 +381,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const uint32_t* __re
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                                                             size_t n, const uint32_t* __restrict__ offsets,
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in,
+                                                             uint32_t* __restrict__ out, size_t n,
+                                                             const uint32_t* __restrict__ offsets,
                                                              uint32_t* __restrict__ grand_total) {
+  frame_order();
   __shared__ uint32_t smem[64];
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
@@ -406,6 +412,7 @@ constexpr int kScanLoopTiles = 8;
 __global__ void __launch_bounds__(kScanThreads) k_scan_loop(const uint32_t* __restrict__ in,
                                                             uint32_t* __restrict__ out, size_t n,
                                                             uint32_t* __restrict__ grand_total) {
+  frame_order();
   __shared__ uint32_t smem[64];
   uint32_t carry = 0;
   for (size_t tile = 0; tile * kScanTile < n; ++tile) {
@@ -440,22 +447,22 @@ cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, size_t n, uint32_t
   }
   const size_t nb = blocks_for(n);
   if (nb == 1) {
-    k_scan_apply<<<1, kScanThreads, 0, s>>>(in, out, n, nullptr, grand_total);
+    launch_in_frame(k_scan_apply, 1, kScanThreads, 0, s, in, out, n, nullptr, grand_total);
     ++*launches;
     return cudaGetLastError();
   }
   if (nb <= (size_t)kScanLoopTiles) {
-    k_scan_loop<<<1, kScanThreads, 0, s>>>(in, out, n, grand_total);
+    launch_in_frame(k_scan_loop, 1, kScanThreads, 0, s, in, out, n, grand_total);
     ++*launches;
     return cudaGetLastError();
   }
   uint32_t* sums = tmp;
   uint32_t* rest = tmp + nb;
-  k_scan_sums<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, sums);
+  launch_in_frame(k_scan_sums, (unsigned)nb, kScanThreads, 0, s, in, n, sums);
   ++*launches;
   cudaError_t e = scan_exclusive(sums, sums, nb, rest, nullptr, s, launches);
   if (e != cudaSuccess) return e;
-  k_scan_apply<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, sums, grand_total);
+  launch_in_frame(k_scan_apply, (unsigned)nb, kScanThreads, 0, s, in, out, n, sums, grand_total);
   ++*launches;
   return cudaGetLastError();
 }
@@ -499,6 +506,7 @@ __global__ void __launch_bounds__(kEmitTile) k_emit(const uint32_t* __restrict__
                                                     uint32_t* __restrict__ keys, uint32_t* __restrict__ tris,
                                                     size_t capacity, const uint32_t* __restrict__ total,
                                                     uint32_t* err) {
+  frame_order();
   __shared__ uint32_t smem[64];
   if (blockIdx.x == 0 && threadIdx.x == 0 && *total > capacity) atomicOr(err, 1u);  // OIT_DEVERR_BIN_OVERFLOW
   const uint32_t t = blockIdx.x * kEmitTile + threadIdx.x;
@@ -541,6 +549,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __
                                                               const uint32_t* __restrict__ total, size_t capacity,
                                                               int shift, size_t chunk, bool digit_major,
                                                               uint32_t* __restrict__ counts) {
+  frame_order();
   __shared__ uint32_t h[kRadixBins];
   h[threadIdx.x] = 0;
   __syncthreads();
@@ -573,6 +582,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
                                                                  const uint32_t* __restrict__ total, size_t capacity,
                                                                  int shift, size_t chunk, uint32_t nchunks,
                                                                  bool scanned, const uint32_t* __restrict__ counts) {
+  frame_order();
   __shared__ uint32_t base[kRadixBins];             // output position of the chunk's next pair of each digit
   __shared__ uint32_t wcount[kSortWarps][kRadixBins];  // per warp: counts, then exclusive offsets in the sub-tile
   __shared__ uint32_t sub_total[kRadixBins];
@@ -677,6 +687,7 @@ __global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* _
                                                               uint32_t* __restrict__ order,
                                                               uint32_t* __restrict__ order_count,
                                                               uint32_t* host_total) {
+  frame_order();
   __shared__ uint32_t first[kListKeys + 1];
   __shared__ uint32_t cnt[2 * kOrderBuckets], base[2 * kOrderBuckets];
   const uint32_t n = (uint32_t)pair_count_of(total, capacity);
@@ -712,10 +723,12 @@ __global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* _
 }
 
 __global__ void k_fill_u32(uint32_t* dst, uint32_t v, size_t n) {
+  frame_order();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) dst[i] = v;
 }
 
 __global__ void k_fill_f4(float4* dst, float4 v, size_t n) {
+  frame_order();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) dst[i] = v;
 }
 
@@ -733,14 +746,14 @@ size_t scan_scratch_words(size_t n) {
 cudaError_t launch_fill_u32(uint32_t* dst, uint32_t value, size_t count, cudaStream_t s) {
   if (!count) return cudaSuccess;
   const unsigned blocks = (unsigned)std::min<size_t>((count + 255) / 256, 152 * 16);
-  k_fill_u32<<<blocks, 256, 0, s>>>(dst, value, count);
+  launch_in_frame(k_fill_u32, blocks, 256, 0, s, dst, value, count);
   return cudaGetLastError();
 }
 
 cudaError_t launch_fill_f4(float4* dst, float4 value, size_t count, cudaStream_t s) {
   if (!count) return cudaSuccess;
   const unsigned blocks = (unsigned)std::min<size_t>((count + 255) / 256, 152 * 16);
-  k_fill_f4<<<blocks, 256, 0, s>>>(dst, value, count);
+  launch_in_frame(k_fill_f4, blocks, 256, 0, s, dst, value, count);
   return cudaGetLastError();
 }
 
@@ -750,11 +763,11 @@ namespace {
 cudaError_t launch_setup(const SetupParams& sp, uint32_t* block_sums, cudaStream_t s, uint64_t* launches) {
   const uint32_t n = sp.num_triangles;
   const int S = sp.samples > 1 ? sp.samples : 1;
-  k_setup<<<(n + 255) / 256, 256, 0, s>>>(sp, S);
+  launch_in_frame(k_setup, (n + 255) / 256, 256, 0, s, sp, S);
   ++*launches;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_setup_clip<<<(unsigned)emit_blocks(n), kClipThreads, 0, s>>>(sp, S, block_sums);
+  launch_in_frame(k_setup_clip, (unsigned)emit_blocks(n), kClipThreads, 0, s, sp, S, block_sums);
   ++*launches;
   return cudaGetLastError();
 }
@@ -807,9 +820,9 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
   cudaError_t e;
   const uint32_t n = sp.num_triangles;
   if (n > 0) {
-    k_emit<<<(unsigned)emit_blocks(n), kEmitTile, 0, s>>>(sp.pair_count, b.pair_offset, b.scan_tmp, sp.bbox, n,
-                                                          sp.tiles_x, sp.opaque_from, (uint32_t)sp.num_tiles, b.keys,
-                                                          b.tris, b.capacity, b.total, error);
+    launch_in_frame(k_emit, (unsigned)emit_blocks(n), kEmitTile, 0, s, sp.pair_count, b.pair_offset, b.scan_tmp,
+                    sp.bbox, n, sp.tiles_x, sp.opaque_from, (uint32_t)sp.num_tiles, b.keys, b.tris, b.capacity,
+                    b.total, error);
     ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   } else if (b.order && (e = cudaMemsetAsync(b.order_count, 0, 2 * kOrderBuckets * 4, s)) != cudaSuccess) {
@@ -820,13 +833,14 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
   uint32_t *kin = b.keys, *vin = b.tris, *kout = b.keys_alt, *vout = b.tris_alt;
   const bool scanned = sort_scanned(b.capacity, b.sort_direct_max);
   for (int shift = 0; shift < key_bits; shift += kRadixBits) {
-    k_radix_hist<<<nchunks, kRadixThreads, 0, s>>>(kin, b.total, b.capacity, shift, chunk, scanned, b.hist);
+    launch_in_frame(k_radix_hist, nchunks, kRadixThreads, 0, s, kin, b.total, b.capacity, shift, chunk, scanned,
+                    b.hist);
     ++*launches;
     if (scanned && (e = scan_exclusive(b.hist, b.hist, (size_t)nchunks * kRadixBins, b.hist + (size_t)nchunks * kRadixBins,
                                        nullptr, s, launches)) != cudaSuccess)
       return e;
-    k_radix_scatter<<<nchunks, kRadixThreads, 0, s>>>(kin, vin, kout, vout, b.total, b.capacity, shift, chunk,
-                                                      nchunks, scanned, b.hist);
+    launch_in_frame(k_radix_scatter, nchunks, kRadixThreads, 0, s, kin, vin, kout, vout, b.total, b.capacity, shift,
+                    chunk, nchunks, scanned, b.hist);
     ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     std::swap(kin, kout);
@@ -837,9 +851,9 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
     std::swap(b.tris, b.tris_alt);
   }
   // ranges of both kinds: [0, num_tiles) opaque, [num_tiles, 2 num_tiles) transparent
-  k_tile_lists<<<(unsigned)((2 * num_tiles + kListKeys - 1) / kListKeys), kListKeys + 32, 0, s>>>(
-      b.keys, b.total, b.capacity, (uint32_t)num_tiles, b.tile_begin, b.tile_end, b.order, b.order_count,
-      b.host_total);
+  launch_in_frame(k_tile_lists, (unsigned)((2 * num_tiles + kListKeys - 1) / kListKeys), kListKeys + 32, 0, s, b.keys,
+                  b.total, b.capacity, (uint32_t)num_tiles, b.tile_begin, b.tile_end, b.order, b.order_count,
+                  b.host_total);
   ++*launches;
   return cudaGetLastError();
 }
