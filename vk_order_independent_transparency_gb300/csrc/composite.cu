@@ -25,14 +25,15 @@ constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 __device__ __forceinline__ bool dge(uint32_t a, uint32_t b) { return __uint_as_float(a) >= __uint_as_float(b); }
 __device__ __forceinline__ bool dlt(uint32_t a, uint32_t b) { return __uint_as_float(a) < __uint_as_float(b); }
 
-template <int L>
+// Sort array of one pixel; the coverage masks only with coverage records.
+template <int L, bool Cov>
 struct Arr {
-  uint32_t c[L], d[L], m[L];
+  uint32_t c[L], d[L], m[Cov ? L : 1];
 };
 
 // bubbleSort, shaders/oitCompositeDefines.glsl:51-89: swaps on >=.
-template <int L>
-__device__ __forceinline__ void bubble_sort(Arr<L>& a, int n) {
+template <int L, bool Cov>
+__device__ __forceinline__ void bubble_sort(Arr<L, Cov>& a, int n) {
 #pragma unroll
   for (int i = L - 2; i >= 0; --i) {
     if (i <= n - 2) {
@@ -42,7 +43,7 @@ __device__ __forceinline__ void bubble_sort(Arr<L>& a, int n) {
           uint32_t t;
           t = a.c[j]; a.c[j] = a.c[j + 1]; a.c[j + 1] = t;
           t = a.d[j]; a.d[j] = a.d[j + 1]; a.d[j + 1] = t;
-          t = a.m[j]; a.m[j] = a.m[j + 1]; a.m[j + 1] = t;
+          if (Cov) { t = a.m[j]; a.m[j] = a.m[j + 1]; a.m[j + 1] = t; }
         }
       }
     }
@@ -52,20 +53,23 @@ __device__ __forceinline__ void bubble_sort(Arr<L>& a, int n) {
 // insertionSort / insertionSortTail, oitCompositeDefines.glsl:94-139, on a
 // full array of L entries. Returns the evicted entry's colour (the item itself
 // when it is not nearer than the last entry).
-template <int L>
-__device__ __forceinline__ uint32_t insertion_sort_tail(Arr<L>& a, uint32_t ic, uint32_t id, uint32_t im) {
+template <int L, bool Cov>
+__device__ __forceinline__ uint32_t insertion_sort_tail(Arr<L, Cov>& a, uint32_t ic, uint32_t id, uint32_t im) {
   if (!dlt(id, a.d[L - 1])) return ic;
   const uint32_t last = a.c[L - 1];
 #pragma unroll
   for (int i = L - 1; i >= 1; --i) {
     if (dlt(id, a.d[i - 1])) {
-      a.c[i] = a.c[i - 1]; a.d[i] = a.d[i - 1]; a.m[i] = a.m[i - 1];
+      a.c[i] = a.c[i - 1]; a.d[i] = a.d[i - 1];
+      if (Cov) a.m[i] = a.m[i - 1];
     } else if (dlt(id, a.d[i])) {
-      a.c[i] = ic; a.d[i] = id; a.m[i] = im;
+      a.c[i] = ic; a.d[i] = id;
+      if (Cov) a.m[i] = im;
     }
   }
   if (dlt(id, a.d[0])) {
-    a.c[0] = ic; a.d[0] = id; a.m[0] = im;
+    a.c[0] = ic; a.d[0] = id;
+    if (Cov) a.m[0] = im;
   }
   return last;
 }
@@ -84,79 +88,99 @@ struct NodeColour {
   }
 };
 
-template <int L, class Col = PackedColour>
-__device__ __forceinline__ float4 blend_array(const Arr<L>& a, int n, int coverage, int S, Col col = Col()) {
+// With coverage (oitSimple.frag.glsl:142-159): per MSAA sample, the fragments
+// covering it, averaged over the samples. Four samples are blended at a time,
+// so an entry's colour is decoded S / 4 times, not S times.
+template <int L, bool Cov, class Col = PackedColour>
+__device__ __forceinline__ float4 blend_array(const Arr<L, Cov>& a, int n, int S, Col col = Col()) {
   float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (!coverage) {
+  if constexpr (!Cov) {
 #pragma unroll
     for (int i = 0; i < L; ++i)
       if (i < n) blend_under(sum, col(a.c[i]));
     return sum;
-  }
-  // oitSimple.frag.glsl:142-159: per MSAA sample, blend the fragments covering it.
-  for (int s = 0; s < S; ++s) {
-    float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
+  } else {
+#pragma unroll 1
+    for (int s0 = 0; s0 < S; s0 += 4) {
+      float4 sc[4];
 #pragma unroll
-    for (int i = 0; i < L; ++i)
-      if (i < n && ((a.m[i] >> s) & 1u)) blend_under(sc, col(a.c[i]));
-    sum.x += sc.x; sum.y += sc.y; sum.z += sc.z; sum.w += sc.w;
+      for (int s = 0; s < 4; ++s) sc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < L; ++i)
+        if (i < n) {
+          const float4 c = col(a.c[i]);
+          const uint32_t m = a.m[i] >> s0;
+#pragma unroll
+          for (int s = 0; s < 4; ++s)
+            if ((m >> s) & 1u) blend_under(sc[s], c);
+        }
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        sum.x += sc[s].x; sum.y += sc[s].y; sum.z += sc[s].z; sum.w += sc[s].w;
+      }
+    }
+    const float k = 1.0f / (float)S;
+    return make_float4(sum.x * k, sum.y * k, sum.z * k, sum.w * k);
   }
-  const float k = 1.0f / (float)S;
-  return make_float4(sum.x * k, sum.y * k, sum.z * k, sum.w * k);
 }
 
 // Simple / Spinlock / Interlock: oitSimple.frag.glsl:115-169 (the Spinlock and
 // Interlock composites, oitSpinlock.frag.glsl:153-207 and
 // oitInterlock.frag.glsl:384-438, are identical).
-template <int L>
+template <int L, bool Cov>
 __device__ __forceinline__ float4 composite_records(const CompositeParams& p, uint32_t eaux, size_t abase) {
   int n = (int)min(p.aux[eaux], (uint32_t)L);
-  Arr<L> a;
+  Arr<L, Cov> a;
 #pragma unroll
   for (int i = 0; i < L; ++i) {
-    a.c[i] = 0; a.d[i] = 0; a.m[i] = 0;
+    a.c[i] = 0; a.d[i] = 0;
+    if (Cov) a.m[i] = 0;
     if (i < n) {
       const size_t o = abase + (size_t)i * p.P;
-      if (p.coverage) {
+      if (Cov) {
         const uint4 r = reinterpret_cast<const uint4*>(p.abuf)[o];
-        a.c[i] = r.x; a.d[i] = r.y; a.m[i] = r.z;
+        a.c[i] = r.x; a.d[i] = r.y;
+        if (Cov) a.m[i] = r.z;
       } else {
         const uint2 r = reinterpret_cast<const uint2*>(p.abuf)[o];
         a.c[i] = r.x; a.d[i] = r.y;
       }
     }
   }
-  bubble_sort<L>(a, n);
-  return blend_array<L>(a, n, p.coverage, p.S);
+  bubble_sort<L, Cov>(a, n);
+  return blend_array<L, Cov>(a, n, p.S);
 }
 
 // Linked list: oitLinkedList.frag.glsl:106-172. With RGBA32F records (F32)
 // nodes are 32 bytes and the sort arrays carry node indices; colours are
 // fetched when blended.
-template <int L, bool F32>
+template <int L, bool F32, bool Cov>
 __device__ __forceinline__ float4 composite_list(const CompositeParams& p, uint32_t eaux) {
   const uint4* __restrict__ pool = reinterpret_cast<const uint4*>(p.abuf);
   uint32_t off = p.aux[eaux];
   if (off >= p.capacity) off = 0;
   int n = 0;
-  Arr<L> a;
+  Arr<L, Cov> a;
 #pragma unroll
   for (int i = 0; i < L; ++i) {
-    a.c[i] = 0; a.d[i] = 0; a.m[i] = 0;
+    a.c[i] = 0; a.d[i] = 0;
+    if (Cov) a.m[i] = 0;
     if (off != 0 && off < p.capacity) {
       if (F32) {
         const uint4 nd = pool[2 * (size_t)off + 1];  // depth, mask, next
-        a.c[i] = off; a.d[i] = nd.x; a.m[i] = nd.y;
+        a.c[i] = off; a.d[i] = nd.x;
+        if (Cov) a.m[i] = nd.y;
         off = nd.z;
       } else {
         const uint4 nd = pool[off];
-        a.c[i] = nd.x; a.d[i] = nd.y; a.m[i] = nd.z;
+        a.c[i] = nd.x; a.d[i] = nd.y;
+        if (Cov) a.m[i] = nd.z;
         off = nd.w;
       }
       n = i + 1;
     }
   }
-  bubble_sort<L>(a, n);
+  bubble_sort<L, Cov>(a, n);
   float4 tail = make_float4(0.f, 0.f, 0.f, 0.f);
   // Lists built by the COLOR pass strictly decrease in node index; the bound
   // only guards against a list that was never built this frame.
@@ -170,11 +194,11 @@ __device__ __forceinline__ float4 composite_list(const CompositeParams& p, uint3
       const uint4 nd = pool[off];
       ic = nd.x; id = nd.y; im = nd.z; next = nd.w;
     }
-    const uint32_t ev = insertion_sort_tail<L>(a, ic, id, im);
+    const uint32_t ev = insertion_sort_tail<L, Cov>(a, ic, id, im);
     if (p.tail) blend_under(tail, F32 ? NodeColour{pool}(ev) : decode_premult(ev));
     off = next;
   }
-  float4 sum = F32 ? blend_array<L>(a, n, p.coverage, p.S, NodeColour{pool}) : blend_array<L>(a, n, p.coverage, p.S);
+  float4 sum = F32 ? blend_array<L, Cov>(a, n, p.S, NodeColour{pool}) : blend_array<L, Cov>(a, n, p.S);
   blend_under(sum, tail);
   return sum;
 }
@@ -183,17 +207,15 @@ __device__ __forceinline__ float4 composite_list(const CompositeParams& p, uint3
 // the local-array walk (list_walk.cuh), whose register use does not grow with
 // OIT_LAYERS (register arrays of 16 or 32 entries cost one or two resident
 // blocks per SM on a latency-bound pointer chase).
-template <int L, bool F32>
+template <int L, bool F32, bool Cov>
 __device__ __forceinline__ float4 list_pixel(const CompositeParams& p, uint32_t eaux) {
-  if (L <= 8) return composite_list<L, F32>(p, eaux);
-  const uint4* __restrict__ pool = reinterpret_cast<const uint4*>(p.abuf);
-  const uint32_t head = p.aux[eaux];
-  if (p.coverage) {
-    WalkArrays<true> a;
-    return walk_list<F32>(pool, head, p.capacity, L, p.tail, p.S, a);
+  if constexpr (L <= 8) {
+    return composite_list<L, F32, Cov>(p, eaux);
+  } else {
+    const uint4* __restrict__ pool = reinterpret_cast<const uint4*>(p.abuf);
+    WalkArrays<Cov> a;
+    return walk_list<F32>(pool, p.aux[eaux], p.capacity, L, p.tail, p.S, a);
   }
-  WalkArrays<false> a;
-  return walk_list<F32>(pool, head, p.capacity, L, p.tail, p.S, a);
 }
 
 // Loop32: oitLoop.frag.glsl:191-222.
@@ -233,7 +255,10 @@ __device__ __forceinline__ void write_out(const CompositeParams& p, uint32_t o, 
 
 enum Kind { kRecords = 0, kList = 1, kLoop = 2, kLoop64 = 3, kListF32 = 4 };
 
-template <int K, int L>
+// Cov: coverage records (MSAA without sample shading). The sort arrays' masks,
+// their swaps and the per-sample blends are compiled only then (this kernel:
+// Interlock 2560x1440 8x MSAA 234 -> 189 us, Spinlock 800x512 17.7 -> 11.7 us).
+template <int K, int L, bool Cov>
 __global__ void __launch_bounds__(256) k_composite(CompositeParams p) {
   frame_order();
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
@@ -249,8 +274,8 @@ __global__ void __launch_bounds__(256) k_composite(CompositeParams p) {
         const uint32_t eaux = (uint32_t)s * p.P + pixel;
         const size_t abase = (size_t)s * (K == kLoop ? 2 : 1) * p.L * p.P + pixel;
         float4 sum;
-        if (K == kRecords) sum = composite_records<L>(p, eaux, abase);
-        else if (K == kList || K == kListF32) sum = list_pixel<L, K == kListF32>(p, eaux);
+        if (K == kRecords) sum = composite_records<L, Cov>(p, eaux, abase);
+        else if (K == kList || K == kListF32) sum = list_pixel<L, K == kListF32, Cov>(p, eaux);
         else if (K == kLoop) sum = composite_loop(p, abase);
         else sum = composite_loop64(p, abase);
         // composite output over the colour target (which already holds the
@@ -304,19 +329,24 @@ __global__ void __launch_bounds__(256) k_composite_weighted(CompositeParams p) {
   write_out(p, (uint32_t)y * (uint32_t)p.W + (uint32_t)x, make_float4(acc.x * k, acc.y * k, acc.z * k, acc.w * k));
 }
 
-template <int K>
-cudaError_t launch_kind(const CompositeParams& p, cudaStream_t s) {
+template <int K, bool Cov>
+cudaError_t launch_layers(const CompositeParams& p, cudaStream_t s) {
   const dim3 grid((p.W + 31) / 32, (p.H + 7) / 8), block(256);
   switch (p.L) {
-    case 1: launch_in_frame(k_composite<K, 1>, grid, block, 0, s, p); break;
-    case 2: launch_in_frame(k_composite<K, 2>, grid, block, 0, s, p); break;
-    case 4: launch_in_frame(k_composite<K, 4>, grid, block, 0, s, p); break;
-    case 8: launch_in_frame(k_composite<K, 8>, grid, block, 0, s, p); break;
-    case 16: launch_in_frame(k_composite<K, 16>, grid, block, 0, s, p); break;
-    case 32: launch_in_frame(k_composite<K, 32>, grid, block, 0, s, p); break;
+    case 1: launch_in_frame(k_composite<K, 1, Cov>, grid, block, 0, s, p); break;
+    case 2: launch_in_frame(k_composite<K, 2, Cov>, grid, block, 0, s, p); break;
+    case 4: launch_in_frame(k_composite<K, 4, Cov>, grid, block, 0, s, p); break;
+    case 8: launch_in_frame(k_composite<K, 8, Cov>, grid, block, 0, s, p); break;
+    case 16: launch_in_frame(k_composite<K, 16, Cov>, grid, block, 0, s, p); break;
+    case 32: launch_in_frame(k_composite<K, 32, Cov>, grid, block, 0, s, p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
+}
+
+template <int K>
+cudaError_t launch_kind(const CompositeParams& p, cudaStream_t s) {
+  return p.coverage ? launch_layers<K, true>(p, s) : launch_layers<K, false>(p, s);
 }
 
 }  // namespace
@@ -328,8 +358,8 @@ cudaError_t launch_composite(Alg alg, const CompositeParams& p, cudaStream_t s) 
     case Alg::Spinlock:
     case Alg::Interlock: return launch_kind<kRecords>(p, s);
     case Alg::LinkedList: return p.record_fp32 ? launch_kind<kListF32>(p, s) : launch_kind<kList>(p, s);
-    case Alg::Loop: launch_in_frame(k_composite<kLoop, 1>, grid, block, 0, s, p); return cudaGetLastError();
-    case Alg::Loop64: launch_in_frame(k_composite<kLoop64, 1>, grid, block, 0, s, p); return cudaGetLastError();
+    case Alg::Loop: launch_in_frame(k_composite<kLoop, 1, false>, grid, block, 0, s, p); return cudaGetLastError();
+    case Alg::Loop64: launch_in_frame(k_composite<kLoop64, 1, false>, grid, block, 0, s, p); return cudaGetLastError();
     case Alg::Weighted: launch_in_frame(k_composite_weighted, grid, block, 0, s, p); return cudaGetLastError();
     default: return cudaErrorInvalidValue;
   }
