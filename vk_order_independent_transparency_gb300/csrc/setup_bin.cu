@@ -396,7 +396,7 @@ constexpr int kEmitTile = kClipThreads * kEmitItems;
 // with block_sums, the block's pair count (after clipping) is written there,
 // the first level of the pair-offset scan. pair_count is 16-byte aligned.
 template <int S>
-__global__ void __launch_bounds__(kClipThreads) k_setup_clip(SetupParams p, uint32_t* __restrict__ block_sums) {
+__global__ void __launch_bounds__(kClipThreads, 12) k_setup_clip(SetupParams p, uint32_t* __restrict__ block_sums) {
   frame_order();
   __shared__ uint32_t warp_sums[kClipThreads / 32];
   const uint32_t n = p.num_triangles;
@@ -780,13 +780,44 @@ __global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* _
                                                               uint32_t* host_total) {
   frame_order();
   __shared__ uint32_t first[kListKeys + 1];
+  __shared__ uint32_t sample[kListKeys], range[2];
   __shared__ uint32_t cnt[2 * kOrderBuckets], base[2 * kOrderBuckets];
   const uint32_t n = (uint32_t)pair_count_of(total, capacity);
   const uint32_t k = blockIdx.x * kListKeys + threadIdx.x;
   if (host_total && blockIdx.x == 0 && threadIdx.x == 0) *host_total = *total;
   if (threadIdx.x < 2 * kOrderBuckets) cnt[threadIdx.x] = 0;
+  // Twice, the block narrows the pairs its keys can start in by a factor of 256,
+  // reading 256 of them at once, before each thread searches what is left: a
+  // step of a search in memory is an L2 round trip.
+  uint32_t lo = 0, hi = n;
+#pragma unroll 1
+  for (int level = 0; level < 2; ++level) {
+    const uint32_t step = max((hi - lo + kListKeys - 1) / kListKeys, 1u);
+    if (threadIdx.x < kListKeys) {
+      const uint32_t i = lo + threadIdx.x * step;
+      sample[threadIdx.x] = i < hi ? __ldg(&keys[i]) & kTileKeyMask : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    // the last sample below k is before k's first pair, the one after it is not
+    uint32_t a = 0, c = kListKeys;
+    while (a < c) {
+      const uint32_t mid = (a + c) >> 1;
+      if (sample[mid] < k) a = mid + 1; else c = mid;
+    }
+    const uint32_t klo = a ? lo + (a - 1) * step : lo, khi = min(lo + a * step, hi);
+    if (level == 0) {
+      if (threadIdx.x == 0) range[0] = klo;
+      if (threadIdx.x == kListKeys) range[1] = khi;
+      __syncthreads();
+      lo = range[0];
+      hi = range[1];
+      __syncthreads();
+    } else {
+      lo = klo;
+      hi = khi;
+    }
+  }
   if (threadIdx.x <= kListKeys) {
-    uint32_t lo = 0, hi = n;
     while (lo < hi) {
       const uint32_t mid = (lo + hi) >> 1;
       if ((__ldg(&keys[mid]) & kTileKeyMask) < k) lo = mid + 1; else hi = mid;
