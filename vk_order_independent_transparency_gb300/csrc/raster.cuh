@@ -1140,6 +1140,9 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
               const uint32_t* odp = p.depth + (size_t)(w.ry0 + dy) * p.RW + (w.rx0 + dx);
               // opaque depth, from memory (in the owner lane it would take S registers)
               auto opaque_depth = [&](int s) { return p.has_opaque ? __ldg(odp + (size_t)s * p.P) : 0x3F800000u; };
+              // without an opaque pass, and with every vertex well in front of depth
+              // 1, every covered sample passes: its depth lies between the vertices'
+              const bool near = !p.has_opaque && zc.x + fmaxf(fmaxf(zc.y, zc.z), 0.0f) < 0.999f;
               if (!(h.x >> 31)) {
                 const int E0 = a.x + b.x * dx + b.y * dy, E1 = a.y + b.z * dx + b.w * dy;
 #pragma unroll
@@ -1148,7 +1151,9 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
                   const int e0 = E0 + (b.x >> 8) * sp.x + (b.y >> 8) * sp.y;
                   const int e1 = E1 + (b.z >> 8) * sp.x + (b.w >> 8) * sp.y;
                   const int e2 = a.z - e0 - e1;
-                  if ((e0 | e1 | e2) >= 0) {
+                  if (near) {
+                    cover |= ((uint32_t)~(e0 | e1 | e2) >> 31) << s;
+                  } else if ((e0 | e1 | e2) >= 0) {
                     const float z = depth_from(zc, to_float((e1 + 1) >> 1), to_float((e2 + 1) >> 1));
                     if (__float_as_uint(z) < opaque_depth(s)) cover |= 1u << s;
                   }
