@@ -258,36 +258,54 @@ enum Kind { kRecords = 0, kList = 1, kLoop = 2, kLoop64 = 3, kListF32 = 4 };
 // Cov: coverage records (MSAA without sample shading). The sort arrays' masks,
 // their swaps and the per-sample blends are compiled only then (this kernel:
 // Interlock 2560x1440 8x MSAA 234 -> 189 us, Spinlock 800x512 17.7 -> 11.7 us).
-template <int K, int L, bool Cov>
+// Sub: the 2x2 supersampled pixels, or the samples of sample shading, that make
+// an output pixel, one lane each (with both modes' products of one, Sub = 1):
+// one thread walking four or eight lists or k-buffers in turn left the kernel
+// waiting on their loads. Their colours are added in the same order.
+template <int K, int L, bool Cov, int Sub>
 __global__ void __launch_bounds__(256) k_composite(CompositeParams p) {
   frame_order();
-  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (x >= p.W || y >= p.H) return;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int dy = 0; dy < p.ss; ++dy)
-    for (int dx = 0; dx < p.ss; ++dx) {
-      const uint32_t pixel = (uint32_t)(y * p.ss + dy) * (uint32_t)p.RW + (uint32_t)(x * p.ss + dx);
-      // one composite per pixel, or per sample with sample shading (each
-      // sample has its own A-buffer at viewSize * layers * sampleID)
-      for (int s = 0; s < p.ssn; ++s) {
-        const uint32_t eaux = (uint32_t)s * p.P + pixel;
-        const size_t abase = (size_t)s * (K == kLoop ? 2 : 1) * p.L * p.P + pixel;
-        float4 sum;
-        if (K == kRecords) sum = composite_records<L, Cov>(p, eaux, abase);
-        else if (K == kList || K == kListF32) sum = list_pixel<L, K == kListF32, Cov>(p, eaux);
-        else if (K == kLoop) sum = composite_loop(p, abase);
-        else sum = composite_loop64(p, abase);
-        // composite output over the colour target (which already holds the
-        // tail-blended opaque + background colour, sample-averaged unless
-        // sample shading keeps one per sample)
-        float4 c = load_color(p.color, p.color_half != 0, eaux);
-        rop_over(c, sum);
-        acc.x += c.x; acc.y += c.y; acc.z += c.z; acc.w += c.w;
-      }
+  // a block's outputs: 32 wide, 8 / Sub rows
+  const int sub = threadIdx.x % Sub, q = threadIdx.x / Sub;
+  const int x = blockIdx.x * 32 + (q & 31);
+  const int y = blockIdx.y * (8 / Sub) + (q >> 5);
+  const bool valid = x < p.W && y < p.H;
+  if (Sub == 1 && !valid) return;
+  float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (valid) {
+    const int s = Sub > 1 && p.ssn > 1 ? sub : 0;
+    const int dx = Sub > 1 && p.ssn == 1 ? sub & 1 : 0, dy = Sub > 1 && p.ssn == 1 ? sub >> 1 : 0;
+    const uint32_t pixel = (uint32_t)(y * p.ss + dy) * (uint32_t)p.RW + (uint32_t)(x * p.ss + dx);
+    // one composite per pixel, or per sample with sample shading (each
+    // sample has its own A-buffer at viewSize * layers * sampleID)
+    const uint32_t eaux = (uint32_t)s * p.P + pixel;
+    const size_t abase = (size_t)s * (K == kLoop ? 2 : 1) * p.L * p.P + pixel;
+    float4 sum;
+    if (K == kRecords) sum = composite_records<L, Cov>(p, eaux, abase);
+    else if (K == kList || K == kListF32) sum = list_pixel<L, K == kListF32, Cov>(p, eaux);
+    else if (K == kLoop) sum = composite_loop(p, abase);
+    else sum = composite_loop64(p, abase);
+    // composite output over the colour target (which already holds the
+    // tail-blended opaque + background colour, sample-averaged unless
+    // sample shading keeps one per sample)
+    c = load_color(p.color, p.color_half != 0, eaux);
+    rop_over(c, sum);
+  }
+  if (Sub > 1) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int first = (int)(threadIdx.x & 31u) - sub;
+#pragma unroll
+    for (int i = 0; i < Sub; ++i) {
+      acc.x += __shfl_sync(0xffffffffu, c.x, first + i);
+      acc.y += __shfl_sync(0xffffffffu, c.y, first + i);
+      acc.z += __shfl_sync(0xffffffffu, c.z, first + i);
+      acc.w += __shfl_sync(0xffffffffu, c.w, first + i);
     }
-  const float k = 1.0f / (float)(p.ss * p.ss * p.ssn);
-  write_out(p, (uint32_t)y * (uint32_t)p.W + (uint32_t)x, make_float4(acc.x * k, acc.y * k, acc.z * k, acc.w * k));
+    const float k = 1.0f / (float)Sub;
+    c = make_float4(acc.x * k, acc.y * k, acc.z * k, acc.w * k);
+    if (!valid || sub) return;
+  }
+  write_out(p, (uint32_t)y * (uint32_t)p.W + (uint32_t)x, c);
 }
 
 // WBOIT composite: oitWeighted.frag.glsl:98-108 with blend
@@ -329,16 +347,20 @@ __global__ void __launch_bounds__(256) k_composite_weighted(CompositeParams p) {
   write_out(p, (uint32_t)y * (uint32_t)p.W + (uint32_t)x, make_float4(acc.x * k, acc.y * k, acc.z * k, acc.w * k));
 }
 
-template <int K, bool Cov>
+template <int K, bool Cov, int Sub>
 cudaError_t launch_layers(const CompositeParams& p, cudaStream_t s) {
-  const dim3 grid((p.W + 31) / 32, (p.H + 7) / 8), block(256);
+  const dim3 grid((p.W + 31) / 32, (p.H + 8 / Sub - 1) / (8 / Sub)), block(256);
+  if constexpr (K == kLoop || K == kLoop64) {  // no sort array
+    launch_in_frame(k_composite<K, 1, Cov, Sub>, grid, block, 0, s, p);
+    return cudaGetLastError();
+  }
   switch (p.L) {
-    case 1: launch_in_frame(k_composite<K, 1, Cov>, grid, block, 0, s, p); break;
-    case 2: launch_in_frame(k_composite<K, 2, Cov>, grid, block, 0, s, p); break;
-    case 4: launch_in_frame(k_composite<K, 4, Cov>, grid, block, 0, s, p); break;
-    case 8: launch_in_frame(k_composite<K, 8, Cov>, grid, block, 0, s, p); break;
-    case 16: launch_in_frame(k_composite<K, 16, Cov>, grid, block, 0, s, p); break;
-    case 32: launch_in_frame(k_composite<K, 32, Cov>, grid, block, 0, s, p); break;
+    case 1: launch_in_frame(k_composite<K, 1, Cov, Sub>, grid, block, 0, s, p); break;
+    case 2: launch_in_frame(k_composite<K, 2, Cov, Sub>, grid, block, 0, s, p); break;
+    case 4: launch_in_frame(k_composite<K, 4, Cov, Sub>, grid, block, 0, s, p); break;
+    case 8: launch_in_frame(k_composite<K, 8, Cov, Sub>, grid, block, 0, s, p); break;
+    case 16: launch_in_frame(k_composite<K, 16, Cov, Sub>, grid, block, 0, s, p); break;
+    case 32: launch_in_frame(k_composite<K, 32, Cov, Sub>, grid, block, 0, s, p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -346,7 +368,17 @@ cudaError_t launch_layers(const CompositeParams& p, cudaStream_t s) {
 
 template <int K>
 cudaError_t launch_kind(const CompositeParams& p, cudaStream_t s) {
-  return p.coverage ? launch_layers<K, true>(p, s) : launch_layers<K, false>(p, s);
+  // (supersampling and sample shading are separate modes, and neither has
+  // coverage records)
+  switch (p.ss * p.ss * p.ssn) {
+    case 1:
+      if constexpr (K != kLoop && K != kLoop64)
+        if (p.coverage) return launch_layers<K, true, 1>(p, s);
+      return launch_layers<K, false, 1>(p, s);
+    case 4: return launch_layers<K, false, 4>(p, s);
+    case 8: return launch_layers<K, false, 8>(p, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 }  // namespace
@@ -358,8 +390,8 @@ cudaError_t launch_composite(Alg alg, const CompositeParams& p, cudaStream_t s) 
     case Alg::Spinlock:
     case Alg::Interlock: return launch_kind<kRecords>(p, s);
     case Alg::LinkedList: return p.record_fp32 ? launch_kind<kListF32>(p, s) : launch_kind<kList>(p, s);
-    case Alg::Loop: launch_in_frame(k_composite<kLoop, 1, false>, grid, block, 0, s, p); return cudaGetLastError();
-    case Alg::Loop64: launch_in_frame(k_composite<kLoop64, 1, false>, grid, block, 0, s, p); return cudaGetLastError();
+    case Alg::Loop: return launch_kind<kLoop>(p, s);
+    case Alg::Loop64: return launch_kind<kLoop64>(p, s);
     case Alg::Weighted: launch_in_frame(k_composite_weighted, grid, block, 0, s, p); return cudaGetLastError();
     default: return cudaErrorInvalidValue;
   }
