@@ -82,7 +82,7 @@ struct SimplePolicy {
   static constexpr bool kViewZ = false;
   static __host__ __device__ size_t smem_bytes_per_warp(int, int, int = 0) { return 0; }
   // the colours and coverage that tail blending takes
-  static __host__ __device__ int payload_bytes(int tail, int) { return tail ? 20 : 0; }
+  static __host__ __device__ int payload_bytes(int tail, int, int) { return tail ? 20 : 0; }
   uint32_t count;
   uint32_t eaux;
   __device__ void init(const RasterParams& p, void*, int, int sample, uint32_t pixel) {
@@ -121,7 +121,7 @@ struct LinkedListPolicy {
   static constexpr bool kDirect = true;
   static constexpr bool kPack = true;
   static __host__ __device__ size_t smem_bytes_per_warp(int, int, int = 0) { return 0; }
-  static __host__ __device__ int payload_bytes(int, int) { return 0; }
+  static __host__ __device__ int payload_bytes(int, int, int) { return 0; }
   uint32_t head;
   uint32_t eaux;
   __device__ void init(const RasterParams& p, void*, int, int sample, uint32_t pixel) {
@@ -163,7 +163,7 @@ struct Loop64Policy {
   static __host__ __device__ size_t smem_bytes_per_warp(int L, int, int fp32 = 0) {
     return (size_t)L * 32 * (fp32 ? 24 : 8);
   }
-  static __host__ __device__ int payload_bytes(int, int fp32) { return fp32 ? 20 : 4; }
+  static __host__ __device__ int payload_bytes(int, int fp32, int) { return fp32 ? 20 : 4; }
   unsigned long long* kb;
   float4* pay;  // RGBA32F payload moving with its key, or null
   int lane, count;
@@ -256,7 +256,7 @@ struct LoopPolicy {
   static constexpr int kWarpsPerSM = 32;
   static constexpr bool kViewZ = false;
   static __host__ __device__ size_t smem_bytes_per_warp(int L, int, int = 0) { return (size_t)L * 32 * 8; }
-  static __host__ __device__ int payload_bytes(int tail, int) { return tail ? 20 : 4; }
+  static __host__ __device__ int payload_bytes(int tail, int, int) { return tail ? 20 : 4; }
   uint32_t* dep;
   uint32_t* col;
   int lane;
@@ -327,7 +327,7 @@ struct LockPolicy {
   static __host__ __device__ size_t smem_bytes_per_warp(int L, int coverage, int = 0) {
     return (size_t)L * 32 * (coverage ? 16 : 8);
   }
-  static __host__ __device__ int payload_bytes(int tail, int) { return tail ? 20 : 4; }
+  static __host__ __device__ int payload_bytes(int tail, int, int) { return tail ? 20 : 4; }
   uint32_t count, auxdepth;
   // the furthest record of a full k-buffer, searched again once it is replaced
   uint32_t maxDepth;
@@ -426,7 +426,7 @@ struct WeightedPolicy {
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = true;
   static __host__ __device__ size_t smem_bytes_per_warp(int, int, int = 0) { return 0; }
-  static __host__ __device__ int payload_bytes(int, int) { return 20; }
+  static __host__ __device__ int payload_bytes(int, int, int weighted_fp32) { return weighted_fp32 ? 20 : 16; }
   // FP16: acc.x and acc.y hold four halves
   float4 acc[S];
   float rev[S];
@@ -731,6 +731,9 @@ __device__ __forceinline__ void walk_pass(const RasterParams& p, const WarpTile&
 //  mine  per 32 queued fragments and lane: the fragments of the lane's pixel;
 //  ring  triangles collected by the walk;
 //  then the policy's payload per queued fragment.
+//  persp WBOIT: the hits' perspective terms. Read from memory per fragment they
+//        were another round trip before it could be shaded: 3840x2160 3.03 ->
+//        2.91 ms, 641x359 86 -> 79 us without it.
 template <bool Samples>
 struct QueueEntry {
   uint32_t depth;
@@ -739,17 +742,18 @@ template <>
 struct QueueEntry<true> {
   uint32_t depth, info;
 };
-template <bool Samples>
+template <bool Samples, bool ViewZ>
 struct WarpStage {
   TriSetup rec[kHits];
   uint2 hit[kHits];
-  QueueEntry<Samples> ent[kQueue];
+  TriPersp persp[ViewZ ? kHits : 1];
+  QueueEntry<Samples> ent[Samples || !ViewZ ? kQueue : 4];  // (WBOIT needs no depths)
   uint32_t mine[kQueue / 32][32];
   uint32_t ring[kRing];
 };
-template <int S>
+template <int S, bool ViewZ>
 __host__ __device__ constexpr size_t warp_stage_bytes(int payload) {
-  return sizeof(WarpStage<(S > 1)>) + (size_t)kQueue * payload;
+  return sizeof(WarpStage<(S > 1), ViewZ>) + (size_t)kQueue * payload;
 }
 
 // Position of set bit n (0 = the lowest) of m; n < popc(m).
@@ -919,14 +923,14 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
   const int warp = threadIdx.x >> 5;
   const WarpTile w = warp_tile<SSN>(p, cta);
   const uint32_t elem = (uint32_t)w.sample * p.P + w.pixel;  // this lane's sample of the pixel
-  const int payload = Pol::payload_bytes(p.tail, p.record_fp32);
-  unsigned char* wbase = smem_raw + (size_t)warp * warp_stage_bytes<S>(payload);
-  using Stage = WarpStage<(S > 1)>;
+  const int payload = Pol::payload_bytes(p.tail, p.record_fp32, p.weighted_fp32);
+  unsigned char* wbase = smem_raw + (size_t)warp * warp_stage_bytes<S, Pol::kViewZ>(payload);
+  using Stage = WarpStage<(S > 1), Pol::kViewZ>;
   Stage& st = *reinterpret_cast<Stage*>(wbase);
   FragPay pay;
   pay.rgba = reinterpret_cast<float4*>(wbase + sizeof(Stage));
   pay.packed = reinterpret_cast<uint32_t*>(wbase + sizeof(Stage) + (payload >= 16 ? kQueue * 16 : 0));
-  unsigned char* pol_smem = smem_raw + (size_t)(blockDim.x >> 5) * warp_stage_bytes<S>(payload) +
+  unsigned char* pol_smem = smem_raw + (size_t)(blockDim.x >> 5) * warp_stage_bytes<S, Pol::kViewZ>(payload) +
                             (size_t)warp * Pol::smem_bytes_per_warp(p.L, p.coverage, p.record_fp32);
 
   PixelTargets<S> tg;
@@ -957,6 +961,11 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
     const bool shading = Pol::kPasses == 1 || pass == Pol::kPasses - 1;
 
     auto stage = [&](uint32_t head, int nh, int& total) {
+      if (Pol::kViewZ && w.lane < nh) {  // (waited for with the records)
+        const TriPersp* src = persp + st.ring[(head + w.lane) % kRing];
+        cp_async16(&st.persp[w.lane].q, &src->q);
+        cp_async16(&st.persp[w.lane].vzq, &src->vzq);
+      }
       return stage_hits<S, SSN, true>(w, setup, st.ring, st.rec, st.hit, lanes, head, nh, total);
     };
 
@@ -985,9 +994,9 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
     };
 
     // Shading of record T from its edge values.
-    auto shade_fragment = [&](uint2 h, uint32_t head, const TriSetup& T, float3 v, Frag& f, Shade& sh) {
+    auto shade_fragment = [&](uint2 h, const TriSetup& T, float3 v, Frag& f, Shade& sh) {
       const int k = (int)((h.x >> 11) & 31u);
-      sh = shade_at(T, v.x, v.y, v.z, Pol::kViewZ ? persp + st.ring[(head + k) % kRing] : nullptr);
+      sh = shade_at(T, v.x, v.y, v.z, Pol::kViewZ ? &st.persp[k] : nullptr);
       f.packed = Pol::kPack ? pack_rgba8(sh, (h.x >> 16) & 255u) : 0u;
     };
 
@@ -1065,12 +1074,12 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
       while (m) {
         const int j = __ffsll((long long)m) - 1;
         m &= m - 1;
-        const auto e = st.ent[j];
+        const auto e = st.ent[Pol::kViewZ && S == 1 ? 0 : j];
         Frag f;
         f.depth = e.depth;
         f.cover = 1u;
         if constexpr (S > 1) f.cover = e.info >> 16;
-        f.packed = shading ? pay.packed[j] : 0u;
+        f.packed = shading && (Pol::kPack || p.weighted_fp32) ? pay.packed[j] : 0u;
         if constexpr (!Pol::kDirect) pol.fragment(p, pass, f, pay, j, tg);
       }
       qn = 0;
@@ -1114,15 +1123,15 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
               if constexpr (Pol::kDirect) {
                 uint32_t node0 = 0;
                 if (Pol::kNodes && w.lane == 0) node0 = atomicAdd(p.counter, (uint32_t)__popc(pm));
-                if (pass_z) shade_fragment(h, head, T, v, f, sh);
+                if (pass_z) shade_fragment(h, T, v, f, sh);
                 write_direct(pass_z, pm, owner, f, sh, alpha, node0);
               } else {
                 if (pass_z) {
                   const int e = qn + __popc(pm & lt);
-                  st.ent[e].depth = f.depth;
+                  if (!Pol::kViewZ) st.ent[e].depth = f.depth;
                   atomicOr(&st.mine[e >> 5][owner], 1u << (e & 31));
                   if (shading) {
-                    shade_fragment(h, head, T, v, f, sh);
+                    shade_fragment(h, T, v, f, sh);
                     Pol::produce(p, pay, e, f, sh, alpha);
                   }
                 }
@@ -1206,7 +1215,7 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
               f.cover = (en.info >> 16) & 255u;
               f.depth = en.depth;
               edges(h, T, owner, v, alpha);
-              shade_fragment(h, head, T, v, f, sh);
+              shade_fragment(h, T, v, f, sh);
             }
             if constexpr (Pol::kDirect) {
               write_direct(act, cnt == 32 ? kFull : (1u << cnt) - 1u, owner, f, sh, alpha, node0);
@@ -1431,11 +1440,17 @@ __global__ void __launch_bounds__(32 * kRasterWarpsPerBlock)
 
 namespace oitd {
 
+// Shared memory of a warp of one view's pass.
+template <template <int> class Pol, int S>
+size_t warp_smem_bytes(const RasterParams& p) {
+  return warp_stage_bytes<S, Pol<S>::kViewZ>(Pol<S>::payload_bytes(p.tail, p.record_fp32, p.weighted_fp32)) +
+         Pol<S>::smem_bytes_per_warp(p.L, p.coverage, p.record_fp32);
+}
+
 template <template <int> class Pol, int S, int SSN, int WPSM>
 cudaError_t launch_transparent_w(const RasterParams& p, cudaStream_t s) {
   const size_t smem = (size_t)kRasterWarpsPerBlock *
-                      (warp_stage_bytes<S>(Pol<S>::payload_bytes(p.tail, p.record_fp32)) +
-                       Pol<S>::smem_bytes_per_warp(p.L, p.coverage, p.record_fp32));
+                      warp_smem_bytes<Pol, S>(p);
   if (smem > 48 * 1024) {
     // raise the kernel's dynamic shared memory cap once per device (never
     // while a CUDA graph is being captured after the first frame)
@@ -1471,8 +1486,7 @@ template <template <int> class Pol, int S, int SSN>
 cudaError_t launch_transparent_mv_s(const oit::MvRaster& mv, cudaStream_t s) {
   size_t per_warp = 0;
   for (int i = 0; i < mv.n; ++i)
-    per_warp = std::max(per_warp, warp_stage_bytes<S>(Pol<S>::payload_bytes(mv.v[i].tail, mv.v[i].record_fp32)) +
-                                      Pol<S>::smem_bytes_per_warp(mv.v[i].L, mv.v[i].coverage, mv.v[i].record_fp32));
+    per_warp = std::max(per_warp, warp_smem_bytes<Pol, S>(mv.v[i]));
   const size_t smem = (size_t)kRasterWarpsPerBlock * per_warp;
   if (smem > 48 * 1024) {
     static int cap_set[64] = {};
