@@ -1736,7 +1736,7 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
       std::vector<int> saved(n);
       for (uint32_t i = 0; i < n; ++i) {  // the budget is baked into the captured launches
         saved[i] = views[i].ctx->raster_wpsm;
-        views[i].ctx->raster_wpsm = (int)cfg.warps_per_sm;
+        views[i].ctx->raster_wpsm = cfg.warps_per_sm ? (int)cfg.warps_per_sm : 36;
       }
       int r = batch_capture(b, views, n, s, cfg.multi_view == 1, cfg.lane_order, &ex, &nodes);
       for (uint32_t i = 0; i < n; ++i) views[i].ctx->raster_wpsm = saved[i];

@@ -160,8 +160,8 @@ struct RasterParams {
   // work binning; null = not wanted (1x only)
   uint8_t* lens;
   int lens_stride;               // micro-tiles per row, (RW + 7) / 8
-  // 1x transparent raster register budget: 32 runs the passes compiled for 36
-  // resident warps per SM (56 registers) at 32 (64 registers); 0 = default
+  // resident warps per SM that the 1x transparent raster is compiled for: 36, or
+  // 32 (any other value)
   int warps_per_sm;
 };
 

@@ -76,8 +76,7 @@ struct SimplePolicy {
   static constexpr bool kDirect = true;
   static constexpr bool kPack = true;
   static constexpr int kPasses = 1;
-  // resident warps per SM with one coverage sample per lane (sets the register
-  // budget: 36 -> 56 registers, spill-free or nearly; 32 -> 64 where 56 spills)
+  // the most resident warps per SM it is compiled for (36: 56 registers)
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = false;
   static __host__ __device__ size_t smem_bytes_per_warp(int, int, int = 0) { return 0; }
@@ -113,8 +112,7 @@ struct SimplePolicy {
 template <int S>
 struct LinkedListPolicy {
   static constexpr int kPasses = 1;
-  // resident warps per SM with one coverage sample per lane (sets the register
-  // budget: 36 -> 56 registers, spill-free or nearly; 32 -> 64 where 56 spills)
+  // the most resident warps per SM it is compiled for (36: 56 registers)
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = false;
   static constexpr bool kNodes = true;
@@ -155,8 +153,7 @@ struct Loop64Policy {
   static constexpr bool kDirect = false;
   static constexpr bool kPack = true;
   static constexpr int kPasses = 1;
-  // resident warps per SM with one coverage sample per lane (sets the register
-  // budget: 36 -> 56 registers, spill-free or nearly; 32 -> 64 where 56 spills)
+  // the most resident warps per SM it is compiled for (36: 56 registers)
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = false;
   // keys, plus a float4 colour per slot with RGBA32F records
@@ -251,8 +248,7 @@ struct LoopPolicy {
   static constexpr bool kDirect = false;
   static constexpr bool kPack = true;
   static constexpr int kPasses = 2;
-  // resident warps per SM with one coverage sample per lane (sets the register
-  // budget: 36 -> 56 registers, spill-free or nearly; 32 -> 64 where 56 spills)
+  // the most resident warps per SM it is compiled for (32: 64 registers)
   static constexpr int kWarpsPerSM = 32;
   static constexpr bool kViewZ = false;
   static __host__ __device__ size_t smem_bytes_per_warp(int L, int, int = 0) { return (size_t)L * 32 * 8; }
@@ -320,8 +316,7 @@ struct LockPolicy {
   static constexpr bool kDirect = false;
   static constexpr bool kPack = true;
   static constexpr int kPasses = 1;
-  // resident warps per SM with one coverage sample per lane (sets the register
-  // budget: 36 -> 56 registers, spill-free or nearly; 32 -> 64 where 56 spills)
+  // the most resident warps per SM it is compiled for (36: 56 registers)
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = false;
   static __host__ __device__ size_t smem_bytes_per_warp(int L, int coverage, int = 0) {
@@ -421,8 +416,7 @@ struct WeightedPolicy {
   static constexpr bool kDirect = false;
   static constexpr bool kPack = false;
   static constexpr int kPasses = 1;
-  // resident warps per SM with one coverage sample per lane: 36 (56
-  // registers, a few spills) measured faster than 32 at 3840x2160 (6.84 vs 6.89 ms)
+  // the most resident warps per SM it is compiled for (36: 56 registers)
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = true;
   static __host__ __device__ size_t smem_bytes_per_warp(int, int, int = 0) { return 0; }
@@ -910,10 +904,14 @@ __device__ __forceinline__ int stage_hits(const WarpTile& w, const TriSetup* __r
 // one tile differ in work (2 warps per CTA: the 64-view batch 5.6% faster
 // than 8; Loop64 k-buffers at large OIT_LAYERS pack shared memory better).
 using oit::kRasterWarpsPerBlock;
-// Policy::kWarpsPerSM resident warps per SM for one coverage sample per lane
-// (36 at 56 registers: the 64-view batch 19.28 -> 18.96 ms against 32 at 64;
-// shared memory still limits Loop64 and Loop32 at large OIT_LAYERS), 24 for
-// MSAA lanes, whose per-sample state needs more.
+// Registers: a spilled value comes back from L2 more often than not, since the
+// warps' stages leave L1 a tenth of the SM's memory. At 64 registers (32 warps
+// per SM) nothing or nearly nothing spills, at 56 (36 warps) 16-40 bytes do:
+// Loop64 1920x1080 324 -> 300 us, Spinlock 800x512 186 -> 173 us, a mostly empty
+// Spinlock 1577x1183 2x2 supersampled frame 366 -> 241 us, WBOIT 3840x2160 the
+// same. A batch's tuner may still take 36. MSAA lanes hold more
+// (msaa_warps): at 24 warps with 8 samples Interlock 2560x1440 took 3.08 ms, at
+// 20 2.83, at 16 3.02; at 24 with 4 samples Simple 1283x717 298 us, at 20 301.
 template <template <int> class Policy, int S, int SSN>
 __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, int cta) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1276,11 +1274,18 @@ __device__ __forceinline__ int mv_view(const oit::MvRaster& mv, uint32_t block, 
 }
 
 
+// Resident warps per SM with S samples a lane (WBOIT: accumulators too).
+template <int S>
+constexpr int msaa_warps(bool weighted) {
+  return S == 4 ? (weighted ? 20 : 24) : (weighted ? 16 : 20);
+}
+
 // One view's pass: one CTA per kRasterWarpsPerBlock micro-tile warps, compiled
 // for WPSM resident warps per SM with one coverage sample per lane (the
 // register budget: 36 -> 56 registers, 32 -> 64).
-template <template <int> class Policy, int S, int SSN, int WPSM = Policy<S>::kWarpsPerSM>
-__global__ void __launch_bounds__(32 * kRasterWarpsPerBlock, (S == 1 ? WPSM : 24) / kRasterWarpsPerBlock)
+template <template <int> class Policy, int S, int SSN, int WPSM>
+__global__ void __launch_bounds__(32 * kRasterWarpsPerBlock,
+                                  (S == 1 ? WPSM : msaa_warps<S>(Policy<S>::kViewZ)) / kRasterWarpsPerBlock)
     k_raster_transparent(RasterParams p) {
   frame_order();
   raster_transparent_body<Policy, S, SSN>(p, (int)blockIdx.x);
@@ -1291,7 +1296,8 @@ __global__ void __launch_bounds__(32 * kRasterWarpsPerBlock, (S == 1 ? WPSM : 24
 // machine and small views fill what large ones leave).
 template <template <int> class Policy, int S, int SSN>
 __global__ void __launch_bounds__(32 * kRasterWarpsPerBlock,
-                                  (S == 1 ? Policy<S>::kWarpsPerSM : 24) / kRasterWarpsPerBlock)
+                                  (S == 1 ? Policy<S>::kWarpsPerSM : msaa_warps<S>(Policy<S>::kViewZ)) /
+                                      kRasterWarpsPerBlock)
     k_raster_transparent_mv(const __grid_constant__ oit::MvRaster mv) {
   frame_order();
   int cta;
@@ -1469,15 +1475,14 @@ cudaError_t launch_transparent_w(const RasterParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// p.warps_per_sm 32 runs the 1x rasters whose default budget is 36 resident
-// warps per SM at 32 (64 registers instead of 56); other values, the default.
+// One sample per lane: 32 warps per SM (64 registers), or where p.warps_per_sm
+// asks for 36 and the policy has it, 36 (56 registers, some spilled).
 template <template <int> class Pol, int S, int SSN>
 cudaError_t launch_transparent_s(const RasterParams& p, cudaStream_t s) {
-  constexpr int kDefault = Pol<S>::kWarpsPerSM;
-  if constexpr (S == 1 && SSN == 1 && kDefault != 32) {
-    if (p.warps_per_sm == 32) return launch_transparent_w<Pol, S, SSN, 32>(p, s);
+  if constexpr (S == 1 && SSN == 1 && Pol<S>::kWarpsPerSM != 32) {
+    if (p.warps_per_sm == Pol<S>::kWarpsPerSM) return launch_transparent_w<Pol, S, SSN, Pol<S>::kWarpsPerSM>(p, s);
   }
-  return launch_transparent_w<Pol, S, SSN, kDefault>(p, s);
+  return launch_transparent_w<Pol, S, SSN, 32>(p, s);
 }
 
 // Multi-view launch of one policy: mv.v[0..n) share S / SSN; the dynamic
