@@ -384,7 +384,7 @@ struct oit_context {
     b.capacity = pair_cap;
     // measured: the 64-view batch 18.64 ms at 8M against 18.96 at 1M; a
     // 2560x1440 MSAA-8 frame alone 6.38 ms at 1M against 6.51 at 8M
-    b.sort_direct_max = in_batch ? (8u << 20) : (1u << 20);
+    b.sort_direct_max = in_batch ? (8u << 20) : (1u << 19);
     return b;
   }
 

@@ -648,15 +648,15 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __
   const size_t beg = (size_t)blockIdx.x * chunk;
   const size_t end = beg + chunk < n ? beg + chunk : n;
   const uint32_t lane = threadIdx.x & 31;
-  for (size_t base = beg; base < end; base += kRadixThreads * 4) {
-    uint32_t d[4];
+  for (size_t base = beg; base < end; base += kRadixThreads * 8) {
+    uint32_t d[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 8; ++k) {
       const size_t i = base + (size_t)k * kRadixThreads + threadIdx.x;
       d[k] = i < end ? (__ldg(&keys[i]) >> shift) & (kRadixBins - 1) : kRadixBins;
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 8; ++k) {
       const uint32_t peers = __match_any_sync(0xffffffffu, d[k]);
       if (d[k] < kRadixBins && (__ffs(peers) - 1) == (int)lane) atomicAdd(&h[d[k]], (uint32_t)__popc(peers));
     }
