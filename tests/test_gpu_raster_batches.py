@@ -72,3 +72,29 @@ def test_opaque_draws_accumulate(engine, aa, cuts):
 
     for a, b in zip(targets(cuts), targets((0, 90))):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize('W,H', [(257, 131), (33, 200)])
+@pytest.mark.parametrize('alg', [oit.OIT_SIMPLE, oit.OIT_LINKEDLIST, oit.OIT_LOOP64])
+def test_many_small_triangles(engine, alg, W, H):
+    """Draws large enough for the setup to test micro-tiles (65536 triangles):
+    slivers, triangles from a fraction of a pixel to several tiles, some over
+    the frame's edge, some split by the near plane, a quarter opaque."""
+    n, L = 66000, 8
+    rng = np.random.default_rng(W)
+    v = np.zeros((n, 3, 10), np.float32)
+    centre = rng.uniform(-1.05, 1.05, (n, 1, 2))
+    size = np.exp(rng.uniform(np.log(0.2), np.log(12.0), (n, 1, 1))) * 2.0 / np.array([W, H])
+    size[::500] *= 5.0
+    offset = rng.uniform(-1.0, 1.0, (n, 3, 2))
+    offset[::3, 2] = offset[::3, 1] + 0.1 * rng.uniform(-1.0, 1.0, (len(offset[::3]), 2))  # slivers
+    v[:, :, :2] = centre + size * offset
+    v[:, :, 2] = rng.uniform(0.05, 0.95, (n, 3))
+    v[::50, 0, 2] = -0.3  # across the near plane
+    v[:, :, 3:6] = rng.normal(size=(n, 3, 3))
+    v[:, :, 6:] = rng.random((n, 1, 4))
+    v, i = v.reshape(-1, 10), np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+    kw = dict(oit_layers=L, nodes_per_pixel=200)
+    g = pu.render_gpu(alg, W, H, v, i, 1, scene_data(), 75, **kw)
+    o = pu.render_oracle(alg, W, H, v, i, 1, scene_data(), 75, **kw)
+    pu.check_pair(alg, g, o, W, H, L)

@@ -47,6 +47,7 @@ struct SetupParams {
   void* setup;            // TriSetup records (96 B)
   void* persp;            // TriPersp records (32 B, WBOIT only) or null
   uint32_t* pair_count;   // [num_triangles] tiles overlapped by both halves (0 = culled)
+  uint32_t* micro;        // the 8x4 micro-tiles a record's triangle may cover (setup_bin.cu); null: those of its bbox
   // frame state the setup clears on the way (null: not): the fragment count,
   // the linked list's node counter, the tile order's bucket counts
   unsigned long long* clear_fragments;
