@@ -319,42 +319,41 @@ struct LockPolicy {
   // the most resident warps per SM it is compiled for (36: 56 registers)
   static constexpr int kWarpsPerSM = 36;
   static constexpr bool kViewZ = false;
-  static __host__ __device__ size_t smem_bytes_per_warp(int L, int coverage, int = 0) {
-    return (size_t)L * 32 * (coverage ? 16 : 8);
+  // depths, then colours (and coverage) of the k-buffer, [layer][lane]
+  static constexpr bool kCover = S > 1;  // several samples a lane: coverage records
+  static __host__ __device__ size_t smem_bytes_per_warp(int L, int, int = 0) {
+    return (size_t)L * 32 * (kCover ? 12 : 8);
   }
   static __host__ __device__ int payload_bytes(int tail, int, int) { return tail ? 20 : 4; }
   uint32_t count, auxdepth;
   // the furthest record of a full k-buffer, searched again once it is replaced
   uint32_t maxDepth;
   int furthest;
-  uint32_t* rec;  // [layer][lane] x words
-  int lane, words;
+  uint32_t* dep;
   uint32_t eaux;
   size_t abase;
   __device__ void init(const RasterParams& p, void* smem, int, int sample, uint32_t pixel) {
-    lane = threadIdx.x & 31;
+    dep = reinterpret_cast<uint32_t*>(smem) + (threadIdx.x & 31);
     eaux = (uint32_t)sample * p.P + pixel;
     abase = (size_t)sample * p.L * p.P + pixel;
-    words = p.coverage ? 4 : 2;
-    rec = reinterpret_cast<uint32_t*>(smem);
     count = 0;
     auxdepth = 0xFFFFFFFFu;
     furthest = -1;
     maxDepth = 0;
   }
-  __device__ __forceinline__ uint32_t* slot(int i) const { return rec + ((size_t)i * 32 + lane) * words; }
+  // record i's colour, and with coverage records its coverage after it
+  __device__ __forceinline__ uint32_t* colour(int L, int i) const {
+    return dep + 32 * (L + i) + (kCover ? (int)(threadIdx.x & 31) + 32 * i : 0);
+  }
   static __device__ __forceinline__ void produce(const RasterParams& p, const FragPay& q, int j, const Frag& f,
                                                  const Shade& sh, float alpha) {
     q.packed[j] = f.packed;
     if (p.tail) q.rgba[j] = make_float4(sh.r, sh.g, sh.b, alpha);
   }
-  __device__ __forceinline__ void store(uint32_t* r, const Frag& f) const {
-    r[0] = f.packed;
-    r[1] = f.depth;
-    if (words == 4) {
-      r[2] = f.cover;
-      r[3] = 0u;
-    }
+  __device__ __forceinline__ void store(int L, int i, const Frag& f) const {
+    dep[32 * i] = f.depth;
+    if constexpr (kCover) *reinterpret_cast<uint2*>(colour(L, i)) = make_uint2(f.packed, f.cover);
+    else *colour(L, i) = f.packed;
   }
   __device__ __forceinline__ void fragment(const RasterParams& p, int, const Frag& f, const FragPay& q, int j,
                                            PixelTargets<S>& tg) {
@@ -364,14 +363,14 @@ struct LockPolicy {
     if (f.depth <= auxdepth) {
       const uint32_t old = count++;
       if (old < (uint32_t)L) {
-        store(slot((int)old), f);
+        store(L, (int)old, f);
         return;  // (a blend of nothing)
       }
       if (furthest < 0) {
         furthest = 0;
         maxDepth = 0;
         for (int i = 0; i < L; ++i) {
-          const uint32_t d = slot(i)[1];
+          const uint32_t d = dep[32 * i];
           if (d > maxDepth) {
             maxDepth = d;
             furthest = i;
@@ -379,10 +378,9 @@ struct LockPolicy {
         }
       }
       if (maxDepth > f.depth) {
-        uint32_t* r = slot(furthest);
-        evicted = r[0];
+        evicted = *colour(L, furthest);
         own = false;
-        store(r, f);
+        store(L, furthest, f);
         auxdepth = maxDepth;
         furthest = -1;
       }
@@ -395,13 +393,10 @@ struct LockPolicy {
     p.auxdepth[eaux] = auxdepth;
     const int n = count < (uint32_t)p.L ? (int)count : p.L;
     for (int i = 0; i < n; ++i) {
-      const uint32_t* r = slot(i);
+      const uint32_t* c = colour(p.L, i);
       const size_t o = abase + (size_t)i * p.P;
-      if (words == 4) {
-        reinterpret_cast<uint4*>(p.abuf)[o] = make_uint4(r[0], r[1], r[2], r[3]);
-      } else {
-        reinterpret_cast<uint2*>(p.abuf)[o] = make_uint2(r[0], r[1]);
-      }
+      if constexpr (kCover) reinterpret_cast<uint4*>(p.abuf)[o] = make_uint4(c[0], dep[32 * i], c[1], 0u);
+      else reinterpret_cast<uint2*>(p.abuf)[o] = make_uint2(c[0], dep[32 * i]);
     }
   }
 };
