@@ -98,3 +98,22 @@ def test_many_small_triangles(engine, alg, W, H):
     g = pu.render_gpu(alg, W, H, v, i, 1, scene_data(), 75, **kw)
     o = pu.render_oracle(alg, W, H, v, i, 1, scene_data(), 75, **kw)
     pu.check_pair(alg, g, o, W, H, L)
+
+
+@pytest.mark.parametrize('tail', [True, False])
+@pytest.mark.parametrize('L', [1, 2, 16, 32])
+@pytest.mark.parametrize('aa', [oit.OIT_AA_NONE, oit.OIT_AA_MSAA_4X, oit.OIT_AA_SSAA_8X])
+def test_loop_second_pass(engine, aa, L, tail):
+    """Loop32 walks a list a second time only where a pixel dropped a fragment:
+    buffers that overflow everywhere, here and there, and nowhere, with equal
+    depths among the triangles."""
+    n, W, H = 120, 21, 13
+    v, i = stack(n, W, H, L, large=True)
+    v = v.reshape(n, 3, 10)
+    v[1::4, :, 2] = 0.5   # equal depths, within and across the kept ones
+    v[3::8, :, 2] = 0.05
+    v = v.reshape(-1, 10)
+    kw = dict(oit_layers=L, aa_type=aa, tail_blend=tail)
+    g = pu.render_gpu(oit.OIT_LOOP, W, H, v, i, 1, scene_data(), 80, **kw)
+    o = pu.render_oracle(oit.OIT_LOOP, W, H, v, i, 1, scene_data(), 80, **kw)
+    pu.check_pair(oit.OIT_LOOP, g, o, W, H, L, aa)
