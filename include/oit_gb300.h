@@ -333,8 +333,8 @@ typedef struct oit_raster_config {
                              1: after every view's binning, one launch per pass, algorithm and sample
                              layout runs the CTAs of all its views, largest views first */
   uint32_t warps_per_sm;  /* register budget of the 1x linked-list, Simple, Loop64 and lock rasters:
-                             36 resident warps per SM (56 registers, the default) or 32 (64 registers;
-                             per-view launches only) */
+                             36 resident warps per SM (56 registers, 0 means this) or 32 (64 registers, which
+                             frames outside a batch use; per-view launches only) */
   int32_t lane_order;     /* how views are spread over the forked streams: 0 round-robin in view order;
                              1 longest first: views in decreasing order of their frame time measured on
                              the batch's first (one by one) frames, each to the stream with the least

@@ -191,9 +191,9 @@ struct oit_context {
       if (e) cudaEventDestroy(e);
     if (scene_ring) cudaFreeHost(scene_ring);
     DevBuf* all[] = {&depth, &opaque_color, &color, &abuf, &aux, &auxdepth, &counter, &accum, &reveal, &out,
-                     &out_linear, &err, &frag, &bbox, &setup, &persp, &pair_count, &micro, &pair_offset, &scan_tmp, &total,
-                     &keys, &tris, &keys_alt, &tris_alt, &hist, &tile_begin, &tile_end, &tile_order, &mesh_v, &mesh_i,
-                     &scene_dev, &lens};
+                     &out_linear, &err, &frag, &bbox, &setup, &persp, &pair_count, &micro, &pair_offset, &scan_tmp,
+                     &total, &keys, &tris, &keys_alt, &tris_alt, &hist, &tile_begin, &tile_end, &tile_order, &mesh_v,
+                     &mesh_i, &scene_dev, &lens};
     for (DevBuf* b : all) b->release();
   }
 
@@ -390,8 +390,11 @@ struct oit_context {
       b.order_count = b.order + order_words();
     }
     b.capacity = pair_cap;
-    // measured: the 64-view batch 18.64 ms at 8M against 18.96 at 1M; a
-    // 2560x1440 MSAA-8 frame alone 6.38 ms at 1M against 6.51 at 8M
+    // 128 chunks or one per 2048 pairs. A frame alone wants every block busy
+    // (512K against 1M: Simple 1283x717 4x MSAA 289 / 297 us, RGBA32F linked
+    // list 700x420 2x2 141 / 145 us); a batch's views fill the GPU together
+    // and want fewer launches (64 views, the sort as it was when the line was
+    // drawn: 18.64 ms at 8M, 18.96 at 1M)
     b.sort_direct_max = in_batch ? (8u << 20) : (1u << 19);
     return b;
   }

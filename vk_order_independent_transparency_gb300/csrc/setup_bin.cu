@@ -639,8 +639,8 @@ cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, size_t n, uint32_t
 // Pair emission: pair j of triangle t lands at pair_offset[t] + j.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t emit_bbox(uint2 bb, uint32_t micro, uint32_t t, uint32_t tile_base, int tiles_x,
-                                              uint32_t off, uint32_t j, uint32_t* __restrict__ keys, uint32_t* __restrict__ tris,
-                                              size_t capacity) {
+                                              uint32_t off, uint32_t j, uint32_t* __restrict__ keys,
+                                              uint32_t* __restrict__ tris, size_t capacity) {
   const int bx0 = bb.x & 0xFFFF, by0 = bb.x >> 16, bx1 = bb.y & 0xFFFF, by1 = (bb.y >> 16) & 0x7FFF;
   if (bx0 > bx1 || by0 > by1) return j;
   const int tx0 = bx0 / kTile, ty0 = by0 / kTile, tx1 = bx1 / kTile, ty1 = by1 / kTile;
@@ -1035,8 +1035,8 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
   const uint32_t n = sp.num_triangles;
   if (n > 0) {
     launch_in_frame(k_emit, (unsigned)emit_blocks(n), kEmitTile, 0, s, sp.pair_count, b.pair_offset, b.scan_tmp,
-                    sp.bbox, sp.micro, n, sp.tiles_x, sp.opaque_from, (uint32_t)sp.num_tiles, b.keys, b.tris, b.capacity,
-                    b.total, error);
+                    sp.bbox, sp.micro, n, sp.tiles_x, sp.opaque_from, (uint32_t)sp.num_tiles, b.keys, b.tris,
+                    b.capacity, b.total, error);
     ++*launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   } else if (b.order && (e = cudaMemsetAsync(b.order_count, 0, 2 * kOrderBuckets * 4, s)) != cudaSuccess) {
@@ -1050,8 +1050,8 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
     launch_in_frame(k_radix_hist, nchunks, kRadixThreads, 0, s, kin, b.total, b.capacity, shift, chunk, scanned,
                     b.hist);
     ++*launches;
-    if (scanned && (e = scan_exclusive(b.hist, b.hist, (size_t)nchunks * kRadixBins, b.hist + (size_t)nchunks * kRadixBins,
-                                       nullptr, s, launches)) != cudaSuccess)
+    const size_t counts = (size_t)nchunks * kRadixBins;
+    if (scanned && (e = scan_exclusive(b.hist, b.hist, counts, b.hist + counts, nullptr, s, launches)) != cudaSuccess)
       return e;
     launch_in_frame(k_radix_scatter, nchunks, kRadixThreads, 0, s, kin, vin, kout, vout, b.total, b.capacity, shift,
                     chunk, nchunks, scanned, b.hist);
