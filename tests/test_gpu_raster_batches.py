@@ -117,3 +117,28 @@ def test_loop_second_pass(engine, aa, L, tail):
     g = pu.render_gpu(oit.OIT_LOOP, W, H, v, i, 1, scene_data(), 80, **kw)
     o = pu.render_oracle(oit.OIT_LOOP, W, H, v, i, 1, scene_data(), 80, **kw)
     pu.check_pair(oit.OIT_LOOP, g, o, W, H, L, aa)
+
+
+@pytest.mark.parametrize('n', [12, 24, 1200])
+def test_sort_chunks(engine, n):
+    """Slivers across the frame, each in thousands of tiles: pairs on both
+    sides of the line (65536) from which a frame's sort sums its chunks' counts
+    in a launch of their own, and more chunks than one round of it takes."""
+    W = H = 1024
+    L = 8
+    rng = np.random.default_rng(n)
+    v = np.zeros((n, 3, 10), np.float32)
+    at = rng.uniform(0.9, 0.99, (n, 2))
+    sign = rng.choice([-1.0, 1.0], n)
+    v[:, 0, 0], v[:, 0, 1] = -at[:, 0], -at[:, 1] * sign
+    v[:, 1, 0], v[:, 1, 1] = at[:, 1], at[:, 0] * sign
+    v[:, 2] = v[:, 1]
+    v[:, 2, 0] += rng.uniform(0.001, 0.003, n)
+    v[:, :, 2] = rng.uniform(0.05, 0.95, (n, 3))
+    v[:, :, 3:6] = rng.normal(size=(n, 3, 3))
+    v[:, :, 6:] = rng.random((n, 1, 4))
+    v, i = v.reshape(-1, 10), np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+    kw = dict(oit_layers=L, nodes_per_pixel=8)
+    g = pu.render_gpu(oit.OIT_LOOP64, W, H, v, i, 1, scene_data(), 100, **kw)
+    o = pu.render_oracle(oit.OIT_LOOP64, W, H, v, i, 1, scene_data(), 100, **kw)
+    pu.check_pair(oit.OIT_LOOP64, g, o, W, H, L)

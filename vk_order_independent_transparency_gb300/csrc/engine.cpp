@@ -390,12 +390,13 @@ struct oit_context {
       b.order_count = b.order + order_words();
     }
     b.capacity = pair_cap;
-    // 128 chunks or one per 2048 pairs. A frame alone wants every block busy
-    // (512K against 1M: Simple 1283x717 4x MSAA 289 / 297 us, RGBA32F linked
-    // list 700x420 2x2 141 / 145 us); a batch's views fill the GPU together
-    // and want fewer launches (64 views, the sort as it was when the line was
-    // drawn: 18.64 ms at 8M, 18.96 at 1M)
-    b.sort_direct_max = in_batch ? (8u << 20) : (1u << 19);
+    // 128 chunks, or one per 2048 pairs and a launch between to sum the
+    // counts. A frame alone wants every block busy (64K / 512K: linked list
+    // 640x480 94 / 98 us, RGBA32F linked list 700x420 2x2 130 / 132, Spinlock
+    // 800x512 147 / 148; smaller ones have few chunks either way); a batch's
+    // views fill the GPU together and want fewer launches (24 views 3.43 ms at
+    // 8M, 3.44 at 1M)
+    b.sort_direct_max = in_batch ? (8u << 20) : (1u << 16);
     return b;
   }
 

@@ -345,7 +345,8 @@ constexpr uint32_t kClipPending = 0xFFFFFFFFu;
 // A warp's records go through shared memory and out in whole 512-byte lines: a
 // thread's own 16-byte stores at a stride of 96 bytes fill half a sector each.
 // With that and 32-bit sample tests of tiny triangles: 983,040 triangles 35 ->
-// 27 us, 15.7 million with WBOIT's records 550 -> 401 us (5.5 TB/s).
+// 27 us, 15.7 million with WBOIT's records 550 -> 401 us (5.5 TB/s; 548 us with
+// the micro-tile test, which saves the raster twice that).
 constexpr int kSetupThreads = 256;
 struct SetupStage {
   uint4 rec[32][7];    // TriSetup, padded: 32 lanes' 16-byte stores in distinct banks
@@ -699,10 +700,11 @@ __global__ void __launch_bounds__(kEmitTile) k_emit(const uint32_t* __restrict__
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort of (key, value) pairs, 8-bit digits.
 //
-// The pairs are cut into at most kSortBlocks chunks (multiples of 2048
-// pairs). k_radix_hist counts each chunk's digits; k_radix_scatter derives
-// its chunk's output offset for every digit from those counts itself (the
-// digit's start over all chunks plus the counts of the chunks before it) and
+// The pairs are cut into chunks: at most kSortBlocks of a multiple of 2048
+// pairs, or any number of 2048. k_radix_hist counts each chunk's digits;
+// k_radix_scatter derives its chunk's output offset for every digit (the
+// digit's start over all chunks plus the counts of the chunks before it) from
+// those counts itself, or from their sums by k_digit_scan, and
 // moves the chunk 2048 pairs at a time: each warp ranks its 256 consecutive
 // pairs with its own shared-memory counters, so a sub-tile costs three block
 // barriers. Pairs keep their order within a digit: the sort is stable.
@@ -716,7 +718,7 @@ constexpr int kSortSubTile = kRadixThreads * kRadixRounds;  // 2048 pairs: 8 war
 constexpr int kSortWarps = kRadixThreads / 32;
 
 // Digit counts of chunk blockIdx.x: counts[chunk * 256 + digit], or, with
-// digit_major (many chunks, scanned in place before the scatter),
+// digit_major (many chunks, summed in place before the scatter),
 // counts[digit * gridDim.x + chunk]. One shared-memory atomic per distinct
 // digit per warp (tile ids of neighbouring pairs are mostly equal).
 __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __restrict__ keys,
@@ -749,6 +751,38 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __
   else counts[(size_t)blockIdx.x * kRadixBins + threadIdx.x] = h[threadIdx.x];
 }
 
+// Running sums, in place, of digit blockIdx.x's counts over the chunks
+// (counts[digit * nchunks + chunk]); the scatter adds the digit's start, the
+// sum of the last ones of the digits before it. A short kernel, bound by its
+// launch and one or two rounds of loads; a scan of the whole array is three of
+// them (Simple 1283x717 4x MSAA, sorting twice, 294 -> 273 us; Spinlock 800x512
+// 155 -> 148; Loop64 1920x1080 286 -> 281).
+constexpr int kDigitScanItems = 8;
+
+__global__ void __launch_bounds__(kRadixThreads) k_digit_scan(uint32_t* __restrict__ counts, uint32_t nchunks) {
+  frame_order();
+  __shared__ uint32_t smem[64];
+  uint32_t* row = counts + (size_t)blockIdx.x * nchunks;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < nchunks; base += kRadixThreads * kDigitScanItems) {
+    const uint32_t first = base + threadIdx.x * kDigitScanItems;
+    uint32_t v[kDigitScanItems], sum = 0;
+#pragma unroll
+    for (int i = 0; i < kDigitScanItems; ++i) {
+      v[i] = first + i < nchunks ? row[first + i] : 0u;
+      sum += v[i];
+    }
+    uint32_t total;
+    uint32_t run = carry + block_exclusive_scan(sum, &total, smem);
+#pragma unroll
+    for (int i = 0; i < kDigitScanItems; ++i) {
+      run += v[i];
+      if (first + i < nchunks) row[first + i] = run;
+    }
+    carry += total;
+  }
+}
+
 __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t* __restrict__ keys_in,
                                                                  const uint32_t* __restrict__ vals_in,
                                                                  uint32_t* __restrict__ keys_out,
@@ -767,9 +801,11 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
   const size_t beg = (size_t)blockIdx.x * chunk;
   // this digit's pairs in all chunks, and in the chunks before this one
   if (scanned) {
-    // the digit-major counts, scanned: this chunk's output offset per digit
-    base[threadIdx.x] = __ldg(&counts[(size_t)threadIdx.x * nchunks + blockIdx.x]);
-    __syncthreads();
+    // the digit-major counts' running sums: of all chunks, and of those before this one
+    const uint32_t* row = counts + (size_t)threadIdx.x * nchunks;
+    const uint32_t before = blockIdx.x ? __ldg(&row[blockIdx.x - 1]) : 0u;
+    uint32_t sum_all;
+    base[threadIdx.x] = block_exclusive_scan(__ldg(&row[nchunks - 1]), &sum_all, scan_s) + before;
   } else {
     // 32 independent loads in flight per thread: the chunks' counts are read
     // by every block, so their latency, not their bytes, is the cost
@@ -989,7 +1025,7 @@ cudaError_t launch_setup(const SetupParams& sp, uint32_t* block_sums, cudaStream
 // Pairs per chunk of the radix sort. Up to direct_max pairs: whole 2048-pair
 // sub-tiles, at most kSortBlocks chunks, each scatter block summing the counts
 // of the chunks before it. Beyond: one sub-tile per chunk (every block busy),
-// the digit-major counts scanned in place.
+// each digit's counts summed over the chunks in place.
 constexpr size_t kSortBlocks = 128;
 bool sort_scanned(size_t capacity, size_t direct_max) { return capacity > direct_max; }
 size_t sort_chunk(size_t capacity, size_t direct_max) {
@@ -1050,9 +1086,10 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
     launch_in_frame(k_radix_hist, nchunks, kRadixThreads, 0, s, kin, b.total, b.capacity, shift, chunk, scanned,
                     b.hist);
     ++*launches;
-    const size_t counts = (size_t)nchunks * kRadixBins;
-    if (scanned && (e = scan_exclusive(b.hist, b.hist, counts, b.hist + counts, nullptr, s, launches)) != cudaSuccess)
-      return e;
+    if (scanned) {
+      launch_in_frame(k_digit_scan, kRadixBins, kRadixThreads, 0, s, b.hist, nchunks);
+      ++*launches;
+    }
     launch_in_frame(k_radix_scatter, nchunks, kRadixThreads, 0, s, kin, vin, kout, vout, b.total, b.capacity, shift,
                     chunk, nchunks, scanned, b.hist);
     ++*launches;
@@ -1072,12 +1109,12 @@ cudaError_t bin_sort(const SetupParams& sp, Bins& b, int key_bits, int num_tiles
   return cudaGetLastError();
 }
 
-// Digit counts of the chunks (and, for the scanned sort, its scan scratch).
+// Digit counts of the chunks.
 size_t radix_hist_words(size_t pairs, bool with_scanned) {
   const size_t direct = kSortBlocks * kRadixBins;
   if (!with_scanned) return direct;
   const size_t words = (pairs + kSortSubTile - 1) / kSortSubTile * kRadixBins;
-  return std::max(direct, words + scan_scratch_words(words));
+  return std::max(direct, words);
 }
 
 void srgb_host_tables(float* thr256, float* dec256) {
