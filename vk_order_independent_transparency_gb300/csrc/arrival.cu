@@ -38,12 +38,12 @@ __device__ __forceinline__ bool locked_tail_blend(const ArrivalParams& p, uint32
       __threadfence();
       float4 c;
       if (p.color_half) {
-        const uint2 v = __ldcg(reinterpret_cast<const uint2*>(p.color) + pixel);
+        const uint2 v = load_cg(reinterpret_cast<const uint2*>(p.color) + pixel);
         const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&v.x));
         const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
         c = make_float4(lo.x, lo.y, hi.x, hi.y);
       } else {
-        c = __ldcg(p.color + pixel);
+        c = load_cg(p.color + pixel);
       }
       rop_over(c, src);
       if (p.color_half) {
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(32 * kArrivalWarps, 4) k_arrival_ll(ArrivalPar
   const uint32_t lt = (1u << lane) - 1u;
   unsigned long long* pre = pre_s[warp];
   uint4* geo = geo_s[warp];
-  const TriSetup* __restrict__ setup = reinterpret_cast<const TriSetup*>(p.setup);
+  const TriSetup* setup = reinterpret_cast<const TriSetup*>(p.setup);
   const uint32_t stride = gridDim.x * kArrivalWarps * 32u;
   uint32_t nfrag = 0;  // warp-uniform
   // entries [0, n): records 0 .. n-1; entries [n, 2n): the second halves of
@@ -80,8 +80,8 @@ __global__ void __launch_bounds__(32 * kArrivalWarps, 4) k_arrival_ll(ArrivalPar
     const uint32_t t = second ? p.second_base + (v - p.num_tris) : v;
     uint32_t x0 = 0, y0 = 0, wd = 1;
     unsigned long long area = 0;
-    if (v < 2u * p.num_tris && (!second || (__ldg(&p.bbox[v - p.num_tris]).y >> 31))) {
-      const uint2 bb = __ldg(&p.bbox[t]);
+    if (v < 2u * p.num_tris && (!second || (p.bbox[v - p.num_tris].y >> 31))) {
+      const uint2 bb = p.bbox[t];
       const int bx0 = bb.x & 0xFFFF, by0 = bb.x >> 16, bx1 = bb.y & 0xFFFF, by1 = (bb.y >> 16) & 0x7FFF;
       if (bx0 <= bx1 && by0 <= by1) {  // culled triangles carry an empty bbox
         x0 = (uint32_t)bx0;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(32 * kArrivalWarps, 4) k_arrival_ll(ArrivalPar
         }
         if (in) {
           pixel = (uint32_t)py * (uint32_t)p.RW + (uint32_t)px;
-          const uint32_t od = p.has_opaque ? __ldg(&p.depth[pixel]) : 0x3F800000u;  // early depth test
+          const uint32_t od = p.has_opaque ? p.depth[pixel] : 0x3F800000u;  // early depth test
           zbits = __float_as_uint(z);
           frag = zbits < od;
         }

@@ -156,7 +156,7 @@ __device__ __forceinline__ float4 composite_records(const CompositeParams& p, ui
 // fetched when blended.
 template <int L, bool F32, bool Cov>
 __device__ __forceinline__ float4 composite_list(const CompositeParams& p, uint32_t eaux) {
-  const uint4* __restrict__ pool = reinterpret_cast<const uint4*>(p.abuf);
+  const uint4* pool = reinterpret_cast<const uint4*>(p.abuf);
   uint32_t off = p.aux[eaux];
   if (off >= p.capacity) off = 0;
   int n = 0;
@@ -212,7 +212,7 @@ __device__ __forceinline__ float4 list_pixel(const CompositeParams& p, uint32_t 
   if constexpr (L <= 8) {
     return composite_list<L, F32, Cov>(p, eaux);
   } else {
-    const uint4* __restrict__ pool = reinterpret_cast<const uint4*>(p.abuf);
+    const uint4* pool = reinterpret_cast<const uint4*>(p.abuf);
     WalkArrays<Cov> a;
     return walk_list<F32>(pool, p.aux[eaux], p.capacity, L, p.tail, p.S, a);
   }
@@ -232,8 +232,8 @@ __device__ __forceinline__ float4 composite_loop(const CompositeParams& p, size_
 // Loop64: oitLoop64.frag.glsl:162-183.
 // With RGBA32F records a float4 payload block follows the keys.
 __device__ __forceinline__ float4 composite_loop64(const CompositeParams& p, size_t abase) {
-  const uint2* __restrict__ ab = reinterpret_cast<const uint2*>(p.abuf);
-  const float4* __restrict__ pay =
+  const uint2* ab = reinterpret_cast<const uint2*>(p.abuf);
+  const float4* pay =
       p.record_fp32 ? reinterpret_cast<const float4*>(ab + (size_t)p.ssn * p.L * p.P) : nullptr;
   float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int i = 0; i < p.L; ++i) {

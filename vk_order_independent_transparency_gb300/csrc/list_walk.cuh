@@ -32,19 +32,19 @@ struct WalkNode {
 // F32: 32-byte nodes (float colour, then depth, mask, next); else 16-byte
 // nodes {rgba8, depth, mask, next}.
 template <bool F32>
-__device__ __forceinline__ WalkNode load_node(const uint4* __restrict__ pool, uint32_t off) {
+__device__ __forceinline__ WalkNode load_node(const uint4* pool, uint32_t off) {
   if (F32) {
-    const uint4 n = __ldg(pool + 2 * (size_t)off + 1);
+    const uint4 n = pool[2 * (size_t)off + 1];
     return WalkNode{off, n.x, n.y, n.z};
   }
-  const uint4 n = __ldg(pool + off);
+  const uint4 n = pool[off];
   return WalkNode{n.x, n.y, n.z, n.w};
 }
 
 template <bool F32>
-__device__ __forceinline__ float4 node_colour(const uint4* __restrict__ pool, uint32_t c) {
+__device__ __forceinline__ float4 node_colour(const uint4* pool, uint32_t c) {
   if (F32) {
-    const uint4 v = __ldg(pool + 2 * (size_t)c);
+    const uint4 v = pool[2 * (size_t)c];
     const float a = __uint_as_float(v.w);
     return make_float4(__uint_as_float(v.x) * a, __uint_as_float(v.y) * a, __uint_as_float(v.z) * a, a);
   }
@@ -54,7 +54,7 @@ __device__ __forceinline__ float4 node_colour(const uint4* __restrict__ pool, ui
 // Node loads straight from the pool; colours decoded with the global tables.
 template <bool F32>
 struct PoolFetch {
-  const uint4* __restrict__ pool;
+  const uint4* pool;
   __device__ __forceinline__ WalkNode operator()(uint32_t off) const { return load_node<F32>(pool, off); }
   __device__ __forceinline__ float4 colour(uint32_t c) const { return node_colour<F32>(pool, c); }
 };
@@ -133,8 +133,8 @@ __device__ __noinline__ void walk_bubble(const Fetch& fetch, uint32_t head, uint
 // reaching OIT_LAYERS nodes (or the end of a shorter list) a flagged array is
 // rebuilt by bubbleSort itself. Later nodes go through insertionSortTail.
 template <bool F32, class A, class Fetch>
-__device__ __forceinline__ void walk_step(ListWalk& w, A& a, const WalkNode& n, const Fetch& fetch,
-                                          const uint4* __restrict__ pool, uint32_t cap, int L, int tail) {
+__device__ __forceinline__ void walk_step(ListWalk& w, A& a, const WalkNode& n, const Fetch& fetch, const uint4* pool,
+                                          uint32_t cap, int L, int tail) {
   constexpr bool Mask = A::kMask;
   const uint32_t next = n.next < cap ? n.next : 0u;
   if (w.k < L) {
@@ -189,8 +189,8 @@ __device__ __forceinline__ void walk_step(ListWalk& w, A& a, const WalkNode& n, 
 // front to back (with coverage: per MSAA sample, the entries covering it,
 // averaged over the S samples, oitSimple.frag.glsl:142-159), then the tail.
 template <bool F32, class A, class Fetch>
-__device__ __forceinline__ float4 walk_list_with(const Fetch& fetch, const uint4* __restrict__ pool, uint32_t head,
-                                                 uint32_t cap, int L, int tail, int S, A& a) {
+__device__ __forceinline__ float4 walk_list_with(const Fetch& fetch, const uint4* pool, uint32_t head, uint32_t cap,
+                                                 int L, int tail, int S, A& a) {
   constexpr bool Mask = A::kMask;
   ListWalk w;
   w.head = head < cap ? head : 0u;
@@ -225,8 +225,8 @@ __device__ __forceinline__ float4 walk_list_with(const Fetch& fetch, const uint4
 }
 
 template <bool F32, class A>
-__device__ __forceinline__ float4 walk_list(const uint4* __restrict__ pool, uint32_t head, uint32_t cap, int L,
-                                            int tail, int S, A& a) {
+__device__ __forceinline__ float4 walk_list(const uint4* pool, uint32_t head, uint32_t cap, int L, int tail, int S,
+                                            A& a) {
   return walk_list_with<F32>(PoolFetch<F32>{pool}, pool, head, cap, L, tail, S, a);
 }
 
@@ -267,8 +267,8 @@ __device__ __forceinline__ void net_sort(uint32_t (&d)[K], uint32_t (&c)[K]) {
 // with equal depths (bubbleSort's order then depends on its passes: the
 // caller's full walk runs it).
 template <int K>
-__device__ __forceinline__ bool walk_list_staged(const uint4* __restrict__ pool, uint32_t head, uint32_t cap,
-                                                 uint32_t* sc, uint32_t* sd, float4& sum) {
+__device__ __forceinline__ bool walk_list_staged(const uint4* pool, uint32_t head, uint32_t cap, uint32_t* sc,
+                                                 uint32_t* sd, float4& sum) {
   constexpr int T = 32;  // the warp's columns: entry i of a lane at [i * 32 + lane]
   uint32_t off = head < cap ? head : 0u;
   int n = 0;

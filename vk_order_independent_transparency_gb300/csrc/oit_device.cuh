@@ -210,6 +210,30 @@ __device__ __forceinline__ void rop_over(float4& dst, const float4& src) {
 
 __device__ __forceinline__ void set_error(uint32_t* err, uint32_t bits) { atomicOr(err, bits); }
 
+// Loads with a cache operator (cs: read once; cg: from L2) of memory that
+// kernels of the frame write. Volatile: the compiler keeps them behind
+// frame_order() (oit_launch.cuh).
+__device__ __forceinline__ uint2 load_cs(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.cs.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_cs(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 load_cg(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.cg.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_cg(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
 // Colour target element: float4, or (OIT_FLAG_HALF_COLOR) four halves.
 __device__ __forceinline__ void store_color(float4* base, bool half, size_t i, float4 c) {
   if (half) {
@@ -224,12 +248,12 @@ __device__ __forceinline__ void store_color(float4* base, bool half, size_t i, f
 // Read once by the composite: streaming loads.
 __device__ __forceinline__ float4 load_color(const float4* base, bool half, size_t i) {
   if (half) {
-    const uint2 v = __ldcs(reinterpret_cast<const uint2*>(base) + i);
+    const uint2 v = load_cs(reinterpret_cast<const uint2*>(base) + i);
     const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&v.x));
     const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
     return make_float4(lo.x, lo.y, hi.x, hi.y);
   }
-  return __ldcs(base + i);
+  return load_cs(base + i);
 }
 
 // Resolved premultiplied colour to the RGBA8 sRGB output (alpha stays

@@ -558,7 +558,7 @@ __device__ __forceinline__ int ordered_tile(const RasterParams& p, int q, int la
   constexpr int B = oit::kOrderBuckets;
   q = (q & 1) ? p.tiles_x * p.tiles_y - 1 - (q >> 1) : q >> 1;
   const int bucket = B - 1 - lane;  // lane 0: the longest lists
-  const uint32_t c = lane < B ? __ldg(&p.order_count[bucket]) : 0u;
+  const uint32_t c = lane < B ? p.order_count[bucket] : 0u;
   uint32_t incl = c;
 #pragma unroll
   for (int o = 1; o < B; o <<= 1) {
@@ -567,7 +567,7 @@ __device__ __forceinline__ int ordered_tile(const RasterParams& p, int q, int la
   }
   const int at = __ffs((int)__ballot_sync(kFull, lane < B && (uint32_t)q < incl)) - 1;
   const uint32_t before = __shfl_sync(kFull, incl - c, at);
-  return (int)__ldg(&p.tile_order[(size_t)(B - 1 - at) * (size_t)(p.tiles_x * p.tiles_y) + ((uint32_t)q - before)]);
+  return (int)p.tile_order[(size_t)(B - 1 - at) * (size_t)(p.tiles_x * p.tiles_y) + ((uint32_t)q - before)];
 }
 
 // cta: the CTA's index within its view's grid.
@@ -653,8 +653,8 @@ __device__ __forceinline__ void walk_list(const RasterParams& p, const WarpTile&
         key[u] = mbit;
         t[u] = (i & 1u) ? p.num_tris + (i >> 1) : (i >> 1);
       } else {
-        key[u] = __ldg(&p.tile_keys[i]);
-        t[u] = __ldg(&p.tile_tris[i]);
+        key[u] = p.tile_keys[i];
+        t[u] = p.tile_tris[i];
       }
     }
   };
@@ -678,8 +678,8 @@ __device__ __forceinline__ void walk_list(const RasterParams& p, const WarpTile&
       for (int u = 0; u < kPer; ++u) {
         if (test && hit[u]) {
           const uint32_t i = at + 32u * u + w.lane;
-          if (ident && (i & 1u) && !(__ldg(&p.bbox[i >> 1]).y >> 31)) hit[u] = false;
-          else if (Fine || ident) hit[u] = bbox_hits(__ldg(&p.bbox[tc[u]]), w);
+          if (ident && (i & 1u) && !(p.bbox[i >> 1].y >> 31)) hit[u] = false;
+          else if (Fine || ident) hit[u] = bbox_hits(p.bbox[tc[u]], w);
           if ((tc[u] >= p.num_tris ? tc[u] - p.num_tris : tc[u]) >= limit) hit[u] = false;
         }
         const uint32_t m = __ballot_sync(kFull, hit[u]);
@@ -705,7 +705,7 @@ __device__ __forceinline__ uint32_t binned_triangles(const RasterParams& p) {
   uint32_t lo = 0, hi = p.num_tris;  // first t with pair_offset[t] + pair_count[t] > capacity
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(&p.pair_offset[mid]) + __ldg(&p.pair_count[mid]) > p.pair_capacity) hi = mid; else lo = mid + 1;
+    if (p.pair_offset[mid] + p.pair_count[mid] > p.pair_capacity) hi = mid; else lo = mid + 1;
   }
   return lo;
 }
@@ -816,7 +816,7 @@ __device__ __forceinline__ uint32_t bbox_lanes(const WarpTile& w, int bx0, int b
 // owner lanes whose pixel exists. Normals: the records' normals and colours
 // are wanted too.
 template <int S, int SSN, bool Normals>
-__device__ __forceinline__ int stage_hits(const WarpTile& w, const TriSetup* __restrict__ setup, const uint32_t* ring,
+__device__ __forceinline__ int stage_hits(const WarpTile& w, const TriSetup* setup, const uint32_t* ring,
                                           TriSetup* rec, uint2* hit, uint32_t lanes, uint32_t head, int nh,
                                           int& total) {
   using M = LaneMap<SSN>;
@@ -832,7 +832,7 @@ __device__ __forceinline__ int stage_hits(const WarpTile& w, const TriSetup* __r
       cp_async16(&dst.n1, &src->n1);
       cp_async16(&dst.n2, &src->n2);
     }
-    const int4 a = __ldg(&src->xy01), b = __ldg(&src->xy2f);
+    const int4 a = src->xy01, b = src->xy2f;
     const int X0 = a.x, Y0 = a.y, X1 = a.z, Y1 = a.w, X2 = b.x, Y2 = b.y;
     const uint32_t flags = (uint32_t)b.z;
     info = ((uint32_t)w.lane << 11) | ((flags << 8) & 0xFF0000u);
@@ -967,8 +967,8 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
 
   const int tile = w.tile + p.tile_offset;
   const uint32_t beg = p.tile_begin[tile], end = p.tile_end[tile];
-  const TriSetup* __restrict__ setup = reinterpret_cast<const TriSetup*>(p.setup);
-  const TriPersp* __restrict__ persp = reinterpret_cast<const TriPersp*>(p.persp);
+  const TriSetup* setup = reinterpret_cast<const TriSetup*>(p.setup);
+  const TriPersp* persp = reinterpret_cast<const TriPersp*>(p.persp);
   const uint32_t lt = (1u << w.lane) - 1u;
   // owner lanes whose pixel exists
   const uint32_t lanes = __ballot_sync(kFull, w.valid);
@@ -1191,7 +1191,7 @@ __device__ __forceinline__ void raster_transparent_body(const RasterParams& p, i
               const int dx = owner % M::kW, dy = owner / M::kW;
               const uint32_t* odp = p.depth + (size_t)(w.ry0 + dy) * p.RW + (w.rx0 + dx);
               // opaque depth, from memory (in the owner lane it would take S registers)
-              auto opaque_depth = [&](int s) { return p.has_opaque ? __ldg(odp + (size_t)s * p.P) : 0x3F800000u; };
+              auto opaque_depth = [&](int s) { return p.has_opaque ? odp[(size_t)s * p.P] : 0x3F800000u; };
               // without an opaque pass, and with every vertex well in front of depth
               // 1, every covered sample passes: its depth lies between the vertices'
               const bool near = !p.has_opaque && zc.x + fmaxf(fmaxf(zc.y, zc.z), 0.0f) < 0.999f;
@@ -1396,7 +1396,7 @@ __device__ __forceinline__ void raster_opaque_body(const RasterParams& p, int ct
   const int warp = threadIdx.x >> 5;
   const WarpTile w = warp_tile<1>(p, cta);
   OpaqueStage<S>& st = st_all[warp];
-  const TriSetup* __restrict__ setup = reinterpret_cast<const TriSetup*>(p.setup);
+  const TriSetup* setup = reinterpret_cast<const TriSetup*>(p.setup);
   const uint32_t lt = (1u << w.lane) - 1u;
   const uint32_t lanes = __ballot_sync(kFull, w.valid);
 #pragma unroll

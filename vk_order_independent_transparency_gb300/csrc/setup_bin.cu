@@ -247,7 +247,7 @@ __device__ __forceinline__ uint32_t setup_half(const SetupParams& p, bool opaque
     return 0;
   }
   T.xy01 = make_int4(PX[0], PY[0], PX[1], PY[1]);
-  float alpha = __fmaf_rn(__ldg(c0 + 3), p.alpha_width, p.alpha_min);
+  float alpha = __fmaf_rn(c0[3], p.alpha_width, p.alpha_min);
   alpha = (alpha > 0.0f) ? alpha : 0.0f;
   alpha = (alpha < 1.0f) ? alpha : 1.0f;
   const int acode = __float2int_rn(__fmul_rn(alpha, 255.0f));
@@ -257,9 +257,9 @@ __device__ __forceinline__ uint32_t setup_half(const SetupParams& p, bool opaque
   const float q0 = q[0], q1 = sw ? q[2] : q[1], q2 = sw ? q[1] : q[2];
   const ClipVert& v1 = sw ? cv[2] : cv[1];
   const ClipVert& v2 = sw ? cv[1] : cv[2];
-  T.n0 = make_float4(__fmul_rn(cv[0].nx, q0), __fmul_rn(cv[0].ny, q0), __fmul_rn(cv[0].nz, q0), __ldg(c0 + 0));
-  T.n1 = make_float4(__fmul_rn(v1.nx, q1), __fmul_rn(v1.ny, q1), __fmul_rn(v1.nz, q1), __ldg(c0 + 1));
-  T.n2 = make_float4(__fmul_rn(v2.nx, q2), __fmul_rn(v2.ny, q2), __fmul_rn(v2.nz, q2), __ldg(c0 + 2));
+  T.n0 = make_float4(__fmul_rn(cv[0].nx, q0), __fmul_rn(cv[0].ny, q0), __fmul_rn(cv[0].nz, q0), c0[0]);
+  T.n1 = make_float4(__fmul_rn(v1.nx, q1), __fmul_rn(v1.ny, q1), __fmul_rn(v1.nz, q1), c0[1]);
+  T.n2 = make_float4(__fmul_rn(v2.nx, q2), __fmul_rn(v2.ny, q2), __fmul_rn(v2.nz, q2), c0[2]);
   if (p.persp) {
     Q.q = make_float4(q0, q1, q2, 0.0f);
     Q.vzq = make_float4(__fmul_rn(cv[0].vz, q0), __fmul_rn(v1.vz, q1), __fmul_rn(v2.vz, q2), 0.0f);
@@ -283,7 +283,7 @@ __device__ __forceinline__ uint32_t setup_half(const SetupParams& p, bool opaque
 // copy of the template is built on the host), colour of the instance.
 __device__ __forceinline__ const float* clip_vertices(const SetupParams& p, uint32_t t, ClipVert (&cv)[3]) {
   const uint32_t tg = p.first_triangle + t;
-  const float* __restrict__ vtx = p.vertices;
+  const float* vtx = p.vertices;
   const float* inst = nullptr;
   uint32_t tri = tg;
   if (p.instances) {
@@ -291,9 +291,9 @@ __device__ __forceinline__ const float* clip_vertices(const SetupParams& p, uint
     tri = tg - o * p.template_triangles;
     inst = p.instances + 8 * (size_t)o;
   }
-  const uint32_t i0 = __ldg(&p.indices[3 * (size_t)tri + 0]);
-  const uint32_t i1 = __ldg(&p.indices[3 * (size_t)tri + 1]);
-  const uint32_t i2 = __ldg(&p.indices[3 * (size_t)tri + 2]);
+  const uint32_t i0 = p.indices[3 * (size_t)tri + 0];
+  const uint32_t i1 = p.indices[3 * (size_t)tri + 1];
+  const uint32_t i2 = p.indices[3 * (size_t)tri + 2];
   const uint32_t vid[3] = {i0, i1, i2};
   // scene constants from device memory (every thread reads the same 80 bytes)
   float m[16], v[16];
@@ -301,7 +301,7 @@ __device__ __forceinline__ const float* clip_vertices(const SetupParams& p, uint
     const float4* sc = reinterpret_cast<const float4*>(p.scene);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float4 c = __ldg(sc + k);
+      const float4 c = sc[k];
       m[4 * k + 0] = c.x;
       m[4 * k + 1] = c.y;
       m[4 * k + 2] = c.z;
@@ -309,14 +309,14 @@ __device__ __forceinline__ const float* clip_vertices(const SetupParams& p, uint
     }
     // of the view matrix only row 2 (view-space z) is used: columns' z entries
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[4 * k + 2] = __ldg(p.scene + 16 + 4 * k + 2);
+    for (int k = 0; k < 4; ++k) v[4 * k + 2] = p.scene[16 + 4 * k + 2];
   }
   float4 ic = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-  if (inst) ic = __ldg(reinterpret_cast<const float4*>(inst));
+  if (inst) ic = *reinterpret_cast<const float4*>(inst);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const float* pv = inst ? vtx + 6 * (size_t)vid[k] : vtx + 10 * (size_t)vid[k];
-    float x = __ldg(pv + 0), y = __ldg(pv + 1), z = __ldg(pv + 2);
+    float x = pv[0], y = pv[1], z = pv[2];
     if (inst) {
       x = __fadd_rn(__fmul_rn(x, ic.w), ic.x);
       y = __fadd_rn(__fmul_rn(y, ic.w), ic.y);
@@ -327,9 +327,9 @@ __device__ __forceinline__ const float* clip_vertices(const SetupParams& p, uint
     cv[k].z = __fmaf_rn(m[2], x, __fmaf_rn(m[6], y, __fmaf_rn(m[10], z, m[14])));
     cv[k].w = __fmaf_rn(m[3], x, __fmaf_rn(m[7], y, __fmaf_rn(m[11], z, m[15])));
     cv[k].vz = __fmaf_rn(v[2], x, __fmaf_rn(v[6], y, __fmaf_rn(v[10], z, v[14])));
-    cv[k].nx = __ldg(pv + 3);
-    cv[k].ny = __ldg(pv + 4);
-    cv[k].nz = __ldg(pv + 5);
+    cv[k].nx = pv[3];
+    cv[k].ny = pv[4];
+    cv[k].nz = pv[5];
   }
   return inst ? inst + 4 : vtx + 10 * (size_t)i0 + 6;  // color.rgba
 }
@@ -474,14 +474,14 @@ constexpr int kEmitTile = kClipThreads * kEmitItems;
 // with block_sums, the block's pair count (after clipping) is written there,
 // the first level of the pair-offset scan. pair_count is 16-byte aligned.
 template <int S>
-__global__ void __launch_bounds__(kClipThreads, 12) k_setup_clip(SetupParams p, uint32_t* __restrict__ block_sums) {
+__global__ void __launch_bounds__(kClipThreads, 12) k_setup_clip(SetupParams p, uint32_t* block_sums) {
   frame_order();
   __shared__ uint32_t warp_sums[kClipThreads / 32];
   const uint32_t n = p.num_triangles;
   const uint32_t t0 = blockIdx.x * kEmitTile + threadIdx.x * kEmitItems;
   uint32_t c[kEmitItems] = {0u, 0u, 0u, 0u};
   if (t0 + 3 < n) {
-    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p.pair_count + t0));
+    const uint4 v = *reinterpret_cast<const uint4*>(p.pair_count + t0);
     c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
   } else {
 #pragma unroll
@@ -536,8 +536,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
   return warp_prefix + x - v;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const uint32_t* __restrict__ in, size_t n,
-                                                            uint32_t* __restrict__ sums) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const uint32_t* in, size_t n, uint32_t* sums) {
   frame_order();
   __shared__ uint32_t smem[64];
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
@@ -550,10 +549,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const uint32_t* __re
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in,
-                                                             uint32_t* __restrict__ out, size_t n,
-                                                             const uint32_t* __restrict__ offsets,
-                                                             uint32_t* __restrict__ grand_total) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in, uint32_t* out, size_t n,
+                                                             const uint32_t* offsets, uint32_t* grand_total) {
   frame_order();
   __shared__ uint32_t smem[64];
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
@@ -578,9 +575,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
 // sum: one launch instead of three for up to kScanLoopTiles tiles.
 constexpr int kScanLoopTiles = 8;
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_loop(const uint32_t* __restrict__ in,
-                                                            uint32_t* __restrict__ out, size_t n,
-                                                            uint32_t* __restrict__ grand_total) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_loop(const uint32_t* in, uint32_t* out, size_t n,
+                                                            uint32_t* grand_total) {
   frame_order();
   __shared__ uint32_t smem[64];
   uint32_t carry = 0;
@@ -640,8 +636,8 @@ cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, size_t n, uint32_t
 // Pair emission: pair j of triangle t lands at pair_offset[t] + j.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t emit_bbox(uint2 bb, uint32_t micro, uint32_t t, uint32_t tile_base, int tiles_x,
-                                              uint32_t off, uint32_t j, uint32_t* __restrict__ keys,
-                                              uint32_t* __restrict__ tris, size_t capacity) {
+                                              uint32_t off, uint32_t j, uint32_t* keys, uint32_t* tris,
+                                              size_t capacity) {
   const int bx0 = bb.x & 0xFFFF, by0 = bb.x >> 16, bx1 = bb.y & 0xFFFF, by1 = (bb.y >> 16) & 0x7FFF;
   if (bx0 > bx1 || by0 > by1) return j;
   const int tx0 = bx0 / kTile, ty0 = by0 / kTile, tx1 = bx1 / kTile, ty1 = by1 / kTile;
@@ -670,20 +666,17 @@ __device__ __forceinline__ uint32_t emit_bbox(uint2 bb, uint32_t micro, uint32_t
 // before it in the block (written to pair_offset, which the bin-overflow walk
 // reads); it emits its first (or only) half's tiles, then the second half's
 // (record n + t) when the near-plane clip split it.
-__global__ void __launch_bounds__(kEmitTile) k_emit(const uint32_t* __restrict__ pair_count,
-                                                    uint32_t* __restrict__ pair_offset,
-                                                    const uint32_t* __restrict__ block_offsets,
-                                                    const uint2* __restrict__ bbox,
-                                                    const uint32_t* __restrict__ micro, uint32_t n, int tiles_x,
-                                                    uint32_t opaque_from, uint32_t num_tiles,
-                                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ tris,
-                                                    size_t capacity, const uint32_t* __restrict__ total,
+__global__ void __launch_bounds__(kEmitTile) k_emit(const uint32_t* pair_count, uint32_t* pair_offset,
+                                                    const uint32_t* block_offsets, const uint2* bbox,
+                                                    const uint32_t* micro, uint32_t n, int tiles_x,
+                                                    uint32_t opaque_from, uint32_t num_tiles, uint32_t* keys,
+                                                    uint32_t* tris, size_t capacity, const uint32_t* total,
                                                     uint32_t* err) {
   frame_order();
   __shared__ uint32_t smem[64];
   if (blockIdx.x == 0 && threadIdx.x == 0 && *total > capacity) atomicOr(err, 1u);  // OIT_DEVERR_BIN_OVERFLOW
   const uint32_t t = blockIdx.x * kEmitTile + threadIdx.x;
-  const uint32_t c = t < n ? __ldg(&pair_count[t]) : 0u;
+  const uint32_t c = t < n ? pair_count[t] : 0u;
   uint32_t block_total;
   const uint32_t off = block_exclusive_scan(c, &block_total, smem) + block_offsets[blockIdx.x];
   if (t >= n) return;
@@ -721,10 +714,9 @@ constexpr int kSortWarps = kRadixThreads / 32;
 // digit_major (many chunks, summed in place before the scatter),
 // counts[digit * gridDim.x + chunk]. One shared-memory atomic per distinct
 // digit per warp (tile ids of neighbouring pairs are mostly equal).
-__global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __restrict__ keys,
-                                                              const uint32_t* __restrict__ total, size_t capacity,
-                                                              int shift, size_t chunk, bool digit_major,
-                                                              uint32_t* __restrict__ counts) {
+__global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* keys, const uint32_t* total,
+                                                              size_t capacity, int shift, size_t chunk,
+                                                              bool digit_major, uint32_t* counts) {
   frame_order();
   __shared__ uint32_t h[kRadixBins];
   h[threadIdx.x] = 0;
@@ -738,7 +730,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const size_t i = base + (size_t)k * kRadixThreads + threadIdx.x;
-      d[k] = i < end ? (__ldg(&keys[i]) >> shift) & (kRadixBins - 1) : kRadixBins;
+      d[k] = i < end ? (keys[i] >> shift) & (kRadixBins - 1) : kRadixBins;
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -759,7 +751,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __
 // 155 -> 148; Loop64 1920x1080 286 -> 281).
 constexpr int kDigitScanItems = 8;
 
-__global__ void __launch_bounds__(kRadixThreads) k_digit_scan(uint32_t* __restrict__ counts, uint32_t nchunks) {
+__global__ void __launch_bounds__(kRadixThreads) k_digit_scan(uint32_t* counts, uint32_t nchunks) {
   frame_order();
   __shared__ uint32_t smem[64];
   uint32_t* row = counts + (size_t)blockIdx.x * nchunks;
@@ -783,13 +775,11 @@ __global__ void __launch_bounds__(kRadixThreads) k_digit_scan(uint32_t* __restri
   }
 }
 
-__global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t* __restrict__ keys_in,
-                                                                 const uint32_t* __restrict__ vals_in,
-                                                                 uint32_t* __restrict__ keys_out,
-                                                                 uint32_t* __restrict__ vals_out,
-                                                                 const uint32_t* __restrict__ total, size_t capacity,
-                                                                 int shift, size_t chunk, uint32_t nchunks,
-                                                                 bool scanned, const uint32_t* __restrict__ counts) {
+__global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t* keys_in, const uint32_t* vals_in,
+                                                                 uint32_t* keys_out, uint32_t* vals_out,
+                                                                 const uint32_t* total, size_t capacity, int shift,
+                                                                 size_t chunk, uint32_t nchunks, bool scanned,
+                                                                 const uint32_t* counts) {
   frame_order();
   __shared__ uint32_t base[kRadixBins];             // output position of the chunk's next pair of each digit
   __shared__ uint32_t wcount[kSortWarps][kRadixBins];  // per warp: counts, then exclusive offsets in the sub-tile
@@ -803,9 +793,9 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
   if (scanned) {
     // the digit-major counts' running sums: of all chunks, and of those before this one
     const uint32_t* row = counts + (size_t)threadIdx.x * nchunks;
-    const uint32_t before = blockIdx.x ? __ldg(&row[blockIdx.x - 1]) : 0u;
+    const uint32_t before = blockIdx.x ? row[blockIdx.x - 1] : 0u;
     uint32_t sum_all;
-    base[threadIdx.x] = block_exclusive_scan(__ldg(&row[nchunks - 1]), &sum_all, scan_s) + before;
+    base[threadIdx.x] = block_exclusive_scan(row[nchunks - 1], &sum_all, scan_s) + before;
   } else {
     // 32 independent loads in flight per thread: the chunks' counts are read
     // by every block, so their latency, not their bytes, is the cost
@@ -814,7 +804,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
     for (uint32_t c0 = 0; c0 < nchunks; c0 += 32) {
       uint32_t v[32];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) v[k] = c0 + k < nchunks ? __ldg(&counts[(size_t)(c0 + k) * kRadixBins + d]) : 0u;
+      for (int k = 0; k < 32; ++k) v[k] = c0 + k < nchunks ? counts[(size_t)(c0 + k) * kRadixBins + d] : 0u;
 #pragma unroll
       for (int k = 0; k < 32; ++k) {
         all += v[k];
@@ -836,8 +826,8 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
 #pragma unroll
     for (int r = 0; r < kRadixRounds; ++r) {
       const size_t i = wbase + (size_t)r * 32 + lane;
-      key[r] = i < end ? __ldg(&keys_in[i]) : 0u;
-      val[r] = i < end ? __ldg(&vals_in[i]) : 0u;
+      key[r] = i < end ? keys_in[i] : 0u;
+      val[r] = i < end ? vals_in[i] : 0u;
     }
 #pragma unroll
     for (int r = 0; r < kRadixRounds; ++r) {
@@ -890,12 +880,9 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
 // lists: order[(kind * kOrderBuckets + bucket) * num_tiles + ...], order_count[kind * kOrderBuckets + bucket].
 constexpr int kListKeys = 256;  // keys per block (of kListKeys + 32 threads)
 
-__global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* __restrict__ keys,
-                                                              const uint32_t* __restrict__ total, size_t capacity,
-                                                              uint32_t num_tiles, uint32_t* __restrict__ begin,
-                                                              uint32_t* __restrict__ end,
-                                                              uint32_t* __restrict__ order,
-                                                              uint32_t* __restrict__ order_count,
+__global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* keys, const uint32_t* total,
+                                                              size_t capacity, uint32_t num_tiles, uint32_t* begin,
+                                                              uint32_t* end, uint32_t* order, uint32_t* order_count,
                                                               uint32_t* host_total) {
   frame_order();
   __shared__ uint32_t first[kListKeys + 1];
@@ -914,7 +901,7 @@ __global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* _
     const uint32_t step = max((hi - lo + kListKeys - 1) / kListKeys, 1u);
     if (threadIdx.x < kListKeys) {
       const uint32_t i = lo + threadIdx.x * step;
-      sample[threadIdx.x] = i < hi ? __ldg(&keys[i]) & kTileKeyMask : 0xFFFFFFFFu;
+      sample[threadIdx.x] = i < hi ? keys[i] & kTileKeyMask : 0xFFFFFFFFu;
     }
     __syncthreads();
     // the last sample below k is before k's first pair, the one after it is not
@@ -939,7 +926,7 @@ __global__ void __launch_bounds__(kListKeys + 32) k_tile_lists(const uint32_t* _
   if (threadIdx.x <= kListKeys) {
     while (lo < hi) {
       const uint32_t mid = (lo + hi) >> 1;
-      if ((__ldg(&keys[mid]) & kTileKeyMask) < k) lo = mid + 1; else hi = mid;
+      if ((keys[mid] & kTileKeyMask) < k) lo = mid + 1; else hi = mid;
     }
     first[threadIdx.x] = lo;
   }
