@@ -118,8 +118,7 @@ struct oit_context {
   size_t tri_cap = 0, pair_cap = 0;
   uint32_t bin_tris = 0, bin_opaque_from = 0;  // the last binned draw: triangles, first opaque one
   bool bin_ordered = false;                    // its tiles are in order of list length
-  bool opaque_valid = false;
-  bool opaque_started = false;  // the frame's opaque targets are written (else its first opaque pass clears them)
+  bool opaque_valid = false;                   // the frame's opaque targets are written, or cleared
   bool color_valid = false;
   int raster_wpsm = 0;  // RasterParams::warps_per_sm of this context's transparent rasters
   cudaStream_t last_stream = nullptr;
@@ -585,7 +584,6 @@ struct oit_context {
   int begin_frame(cudaStream_t s) {
     last_stream = s;
     opaque_valid = false;
-    opaque_started = false;
     color_valid = false;
     return OIT_OK;
   }
@@ -606,7 +604,6 @@ struct oit_context {
     last_stream = s;
     int r = ensure_opaque_buffers();
     if (r != OIT_OK) return r;
-    opaque_valid = true;
     if (!count) return clear_opaque_targets(s);
     cudaEvent_t t0 = prof_begin(s);
     r = bin(mesh, first, count, 0u, s);
@@ -619,28 +616,28 @@ struct oit_context {
   }
 
   int clear_opaque_targets(cudaStream_t s) {
-    if (opaque_started) return OIT_OK;
+    if (opaque_valid) return OIT_OK;
     OIT_TRY_CUDA(oit::launch_fill_u32(depth.as<uint32_t>(), 0x3F800000u, (size_t)S * P, s), "fill");
     OIT_TRY_CUDA(oit::launch_fill_f4(opaque_color.as<float4>(), background, (size_t)S * P, s), "fill");
     launches += 2;
-    opaque_started = true;
+    opaque_valid = true;
     return OIT_OK;
   }
 
-  oit::RasterParams opaque_pass_params() {
+  oit::RasterParams opaque_pass_params(bool fresh) {
     oit::RasterParams p = raster_params(0);
     p.S = S;    // the opaque pass always tests every sample of a pixel
     p.ssn = 1;
-    p.opaque_fresh = opaque_started ? 0 : 1;
+    p.opaque_fresh = fresh ? 1 : 0;
     return p;
   }
 
   int raster_opaque(cudaStream_t s) {
-    oit::RasterParams p = opaque_pass_params();
+    oit::RasterParams p = opaque_pass_params(!opaque_valid);
     cudaEvent_t t1 = prof_begin(s);
     const int r = raster(oit::Alg::Opaque, p, s);
     prof_end(OIT_PROF_OPAQUE_RASTER, t1, s);
-    if (r == OIT_OK) opaque_started = true;
+    if (r == OIT_OK) opaque_valid = true;
     return r;
   }
 
@@ -770,7 +767,6 @@ struct oit_context {
     if (r == OIT_OK && total_tris == 0) r = clear_transparent(s);
     if (r == OIT_OK && num_opaque > 0) r = ensure_opaque_buffers();
     if (r != OIT_OK) return r;
-    opaque_valid = num_opaque > 0;
     cudaEvent_t t0 = prof_begin(s);
     clear_in_setup = true;
     r = bin(mesh, 0, total_tris, nt, s);
@@ -779,7 +775,8 @@ struct oit_context {
     prof_end(OIT_PROF_TRANSPARENT_BIN, t0, s);
     frame_has_opaque = num_opaque > 0;
     if (!raster) {
-      color_valid = true;  // the batch's multi-view rasters follow in the same graph
+      opaque_valid = num_opaque > 0;  // the batch's multi-view rasters follow in the same graph
+      color_valid = true;
       return OIT_OK;
     }
     if (num_opaque > 0) r = raster_opaque(s);
@@ -1262,7 +1259,7 @@ int batch_mv_rasters(const oit_view_frame* views, uint32_t n, cudaStream_t s, ui
     while (k < items.size() && mv->n < oit::kMvMaxViews && items[k].opaque == g.opaque && items[k].alg == g.alg &&
            items[k].S == g.S && items[k].ssn == g.ssn) {
       oit_context* c = items[k].c;
-      mv->v[mv->n] = g.opaque ? c->opaque_pass_params() : c->raster_params(c->num_tiles);
+      mv->v[mv->n] = g.opaque ? c->opaque_pass_params(true) : c->raster_params(c->num_tiles);
       ctas += (uint32_t)(c->tiles_x * c->tiles_y * (g.opaque ? 1 : c->ssn) *
                          (oit::kWarpsPerTile / oit::kRasterWarpsPerBlock));
       mv->cta_end[mv->n++] = ctas;
