@@ -78,3 +78,30 @@ def test_invalid_hook_argument():
     with pytest.raises(oit.OitError) as e:
         oit.debug_fail_allocations(-2)
     assert e.value.status == oit.OIT_ERR_INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize('alg', [oit.OIT_LINKEDLIST, oit.OIT_WEIGHTED])
+@pytest.mark.parametrize('after', range(12))
+def test_smaller_draw_after_a_failed_larger_one(alg, after):
+    """A larger frame fails at any one of the buffers it grows; the smaller
+    frame before it then still renders, and so does the larger one."""
+    W, H = 96, 64
+    kw = dict(oit_layers=8, weighted_precision=oit.OIT_WEIGHTED_FP32)
+    small, large = pu.scene(40, W, H, seed=9), pu.scene(700, W, H, seed=10)
+    refs = [pu.render_gpu(alg, W, H, v, i, tpo, sd, 100, **kw)['image'] for v, i, tpo, sd in (small, large)]
+    meshes = [oit.DeviceMesh(v, i) for v, i, _, _ in (small, large)]
+    tpo, sd = small[2:]
+    r = oit.Renderer(oit.make_state(alg, W, H, **kw))
+    r.update_scene(sd)
+    r.render_frame(meshes[0], tpo, 100)
+    oit.debug_fail_allocations(after)
+    try:
+        r.render_frame(meshes[1], tpo, 100)
+    except oit.OitError as e:
+        assert e.status == oit.OIT_ERR_OUT_OF_MEMORY
+    oit.debug_fail_allocations(-1)
+    for k in (0, 1, 0):
+        r.render_frame(meshes[k], tpo, 100)
+        np.testing.assert_array_equal(r.output(), refs[k])
+    assert r.get_error() == 0
+    r.close()

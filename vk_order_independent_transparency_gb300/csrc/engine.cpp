@@ -287,6 +287,7 @@ struct oit_context {
   int ensure_triangles(size_t n) {
     if (n <= tri_cap) return OIT_OK;
     const size_t cap = std::max<size_t>(n, 1024);
+    tri_cap = 0;  // until every buffer holds `cap`: growing one frees it first
     // two records per triangle: the second half of a triangle the near plane
     // splits lives at record count + t
     OIT_TRY_CUDA(bbox.ensure(2 * cap * 8), "alloc bbox");
@@ -303,6 +304,7 @@ struct oit_context {
     if (n > pair_cap || pair_cap == 0) {
       const float scale = st.bin_capacity_scale > 0.0f ? st.bin_capacity_scale : 1.25f;
       const size_t cap = std::max<size_t>((size_t)((double)n * std::max(1.0f, scale)), 4096);
+      pair_cap = 0;  // as tri_cap
       OIT_TRY_CUDA(keys.ensure(cap * 4), "alloc keys");
       OIT_TRY_CUDA(tris.ensure(cap * 4), "alloc tris");
       OIT_TRY_CUDA(keys_alt.ensure(cap * 4), "alloc keys");
