@@ -82,3 +82,38 @@ def test_opaque_draw_after_a_batch(engine, mode, replays):
         r.draw_opaque(extra, 0, extra.num_triangles)
         for a, b in zip(targets(r), expected(sd, alg, oit.OIT_AA_NONE, mesh, tpo, 60, extra, extra.num_triangles)):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize('staged', [True, False])
+@pytest.mark.parametrize('after', [0, 2])
+def test_failed_opaque_draw_leaves_cleared_targets(engine, staged, after):
+    """A frame (or an opaque draw) that fails for want of memory leaves no
+    earlier frame's opaque content for the draws that follow it."""
+    mesh, tpo, extra, sd = meshes()
+    v, i, big_tpo, _ = pu.scene(400, W, H, seed=8)
+    big = oit.DeviceMesh(v, i)
+    with renderer(sd, oit.OIT_SIMPLE, oit.OIT_AA_NONE) as r:
+        r.render_frame(mesh, tpo, 60)
+        if staged:
+            r.begin_frame()
+            r.clear_transparent()
+        oit.debug_fail_allocations(after)  # among the larger mesh's buffers
+        try:
+            with pytest.raises(oit.OitError) as e:
+                if staged:
+                    r.draw_opaque(big, 0, big.num_triangles)
+                else:
+                    r.render_frame(big, big_tpo, 0)
+        finally:
+            oit.debug_fail_allocations(-1)
+        assert e.value.status == oit.OIT_ERR_OUT_OF_MEMORY
+        depth, color = targets(r)
+        assert depth.size == W * H and (depth == 0x3F800000).all()
+        assert color.size == 4 * W * H and (color.view(np.float32) == np.float32(0.2)).all()
+        r.clear_transparent()
+        r.draw_transparent_color(extra, 0, extra.num_triangles)
+        r.composite()
+        image = r.output()
+    with renderer(sd, oit.OIT_SIMPLE, oit.OIT_AA_NONE) as r:
+        r.render_frame(extra, tpo, 100)
+        np.testing.assert_array_equal(image, r.output())

@@ -640,6 +640,7 @@ struct oit_context {
     const int r = raster(oit::Alg::Opaque, p, s);
     prof_end(OIT_PROF_OPAQUE_RASTER, t1, s);
     if (r == OIT_OK) opaque_valid = true;
+    else clear_opaque_targets(s);
     return r;
   }
 
@@ -773,7 +774,10 @@ struct oit_context {
     clear_in_setup = true;
     r = bin(mesh, 0, total_tris, nt, s);
     clear_in_setup = false;
-    if (r != OIT_OK) return r;
+    if (r != OIT_OK) {
+      if (num_opaque > 0) clear_opaque_targets(s);  // later draws find no earlier frame's
+      return r;
+    }
     prof_end(OIT_PROF_TRANSPARENT_BIN, t0, s);
     frame_has_opaque = num_opaque > 0;
     if (!raster) {
