@@ -1,0 +1,58 @@
+"""Captured frames after their context's buffers have moved: a larger draw, or
+another batch over the same contexts, grows them between two replays."""
+import numpy as np
+import pytest
+
+import parity_util as pu
+import vk_order_independent_transparency_gb300 as oit
+
+pytestmark = pytest.mark.gpu
+
+W, H = 96, 64
+KW = dict(oit_layers=8, nodes_per_pixel=60)
+
+
+def scenes(alg, seed):
+    """[(mesh, triangles per object, scene constants, image)] of a small and a large scene."""
+    out = []
+    for n in (12, 600):
+        v, i, tpo, sd = pu.scene(n, W, H, seed=seed)
+        out.append((oit.DeviceMesh(v, i), tpo, sd, pu.render_gpu(alg, W, H, v, i, tpo, sd, 100, **KW)['image']))
+    return out
+
+
+@pytest.mark.parametrize('alg', [oit.OIT_LINKEDLIST, oit.OIT_SPINLOCK])
+def test_replay_after_a_larger_draw(engine, alg):
+    (mesh, tpo, sd, ref), (large, _, _, large_ref) = scenes(alg, 3)
+    with oit.Renderer(oit.make_state(alg, W, H, flags=oit.OIT_FLAG_CUDA_GRAPH, **KW)) as r:
+        r.update_scene(sd)
+        for _ in range(2):
+            r.render_frame(mesh, tpo, 100)
+            np.testing.assert_array_equal(r.output(), ref)
+        r.begin_frame()
+        r.clear_transparent()
+        r.draw_transparent_color(large, 0, large.num_triangles)
+        r.composite()
+        np.testing.assert_array_equal(r.output(), large_ref)
+        for _ in range(2):
+            r.render_frame(mesh, tpo, 100)
+            np.testing.assert_array_equal(r.output(), ref)
+        assert r.get_error() == 0
+
+
+def test_two_batches_over_the_same_contexts(engine):
+    algs = [oit.OIT_LINKEDLIST, oit.OIT_LOOP64, oit.OIT_SIMPLE]
+    sc = [scenes(alg, 20 + k) for k, alg in enumerate(algs)]
+    renderers = [oit.Renderer(oit.make_state(alg, W, H, **KW)) for alg in algs]
+    batches = []
+    for size in (0, 1):
+        b = oit.Batch(parallel_streams=2)
+        b.set_views([(r, s[size][0], s[size][1], 100) for r, s in zip(renderers, sc)])
+        batches.append(b)
+    for r, s in zip(renderers, sc):
+        r.update_scene(s[0][2])
+    for size in (0, 0, 1, 1, 0, 0, 1):
+        batches[size].render()
+        for r, s in zip(renderers, sc):
+            np.testing.assert_array_equal(r.output(), s[size][3])
+            assert r.get_error() == 0

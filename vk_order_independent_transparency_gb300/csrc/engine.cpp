@@ -7,6 +7,7 @@
 // to the back buffer (copyOffscreenToBackBuffer, main.cpp:645-774). Every
 // entry point returns a status and never aborts.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -34,8 +35,10 @@ std::atomic<int> g_fail_alloc_countdown{-1};
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  uint64_t moves = 0;  // times it was allocated: a captured graph holds the address of one of them
   cudaError_t ensure(size_t n) {
     if (n <= bytes && p) return cudaSuccess;
+    ++moves;
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
@@ -189,11 +192,22 @@ struct oit_context {
     for (cudaEvent_t e : scene_ev)
       if (e) cudaEventDestroy(e);
     if (scene_ring) cudaFreeHost(scene_ring);
-    DevBuf* all[] = {&depth, &opaque_color, &color, &abuf, &aux, &auxdepth, &counter, &accum, &reveal, &out,
-                     &out_linear, &err, &frag, &bbox, &setup, &persp, &pair_count, &micro, &pair_offset, &scan_tmp,
-                     &total, &keys, &tris, &keys_alt, &tris_alt, &hist, &tile_begin, &tile_end, &tile_order, &mesh_v,
-                     &mesh_i, &scene_dev, &lens};
-    for (DevBuf* b : all) b->release();
+    for (DevBuf* b : buffers()) b->release();
+  }
+
+  std::array<DevBuf*, 33> buffers() {
+    return {&depth, &opaque_color, &color, &abuf, &aux, &auxdepth, &counter, &accum, &reveal, &out, &out_linear, &err,
+            &frag, &bbox, &setup, &persp, &pair_count, &micro, &pair_offset, &scan_tmp, &total, &keys, &tris,
+            &keys_alt, &tris_alt, &hist, &tile_begin, &tile_end, &tile_order, &mesh_v, &mesh_i, &scene_dev, &lens};
+  }
+
+  // Grows whenever a buffer is reallocated: a graph captured before that holds
+  // addresses that are no longer the context's. (The sort's buffers change
+  // places, not the sum.)
+  uint64_t buffer_moves() {
+    uint64_t n = 0;
+    for (const DevBuf* b : buffers()) n += b->moves;
+    return n;
   }
 
   oit::Alg alg() const { return static_cast<oit::Alg>(st.algorithm); }
@@ -797,6 +811,7 @@ struct oit_context {
   int32_t debug_held_lock = -1;  // oit_debug_hold_arrival_lock  // binning inside a batch graph, beside other views
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_sig = 0;
+  uint64_t graph_moves = 0;  // buffer_moves() at its capture
   uint64_t graph_launches = 0;
   bool graph_opaque_valid = false;
   std::vector<uint64_t> graph_stats;
@@ -857,8 +872,9 @@ struct oit_context {
                               (uint64_t)(uintptr_t)mesh.instances, mesh.num_triangles, tpo, (uint64_t)percent,
                               (uint64_t)(uintptr_t)out_dev, (uint64_t)(uintptr_t)s};
     for (uint64_t v : parts) sig = (sig ^ v) * 1099511628211ull;
-    // bins that outgrew their capacity since the capture invalidate the graph
-    if (!graph_bins_fit()) drop_graph();
+    // bins that outgrew their capacity since the capture invalidate the graph,
+    // and so do buffers that another draw, or a batch, made grow
+    if (!graph_bins_fit() || graph_moves != buffer_moves()) drop_graph();
     int gr = ensure_graph_stream();
     if (gr != OIT_OK) return gr;
     if (!graph_exec || graph_sig != sig) {
@@ -885,6 +901,7 @@ struct oit_context {
       cudaGraphDestroy(g);
       OIT_TRY_CUDA(ie, "instantiate");
       graph_sig = sig;
+      graph_moves = buffer_moves();
       graph_opaque_valid = opaque_valid;
       graph_launches = launches - l0;
       launches = l0;
@@ -916,6 +933,7 @@ struct oit_batch {
   std::vector<cudaEvent_t> joins;
   cudaGraphExec_t exec = nullptr;
   uint64_t sig = 0;
+  uint64_t moves = 0;  // the views' buffer_moves() at the graph's capture
   uint64_t graph_launches = 0;
   std::vector<oit_context*> ctxs;
   std::vector<bool> opaque_valid;
@@ -1679,9 +1697,14 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
     for (uint64_t x : parts) sig = (sig ^ x) * 1099511628211ull;
   }
   sig ^= n;
+  auto moves = [&] {
+    uint64_t m = 0;
+    for (uint32_t i = 0; i < n; ++i) m += views[i].ctx->buffer_moves();
+    return m;
+  };
   bool fit = true;
   for (uint32_t i = 0; i < n; ++i) fit = views[i].ctx->graph_bins_fit() && fit;
-  if (!fit || sig != b->sig) b->drop();
+  if (!fit || sig != b->sig || moves() != b->moves) b->drop();
   if (!b->exec) {
     // plain frames, one view after the other, size every buffer (and time
     // each view for the longest-first lane order); views the batched resolve
@@ -1777,6 +1800,7 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
     OIT_TRY_CUDA(cudaStreamSynchronize(b->stream), "sync");
     b->exec = best;
     b->sig = sig;
+    b->moves = moves();
     b->graph_launches = best_launches;
     b->raster_cfg = best_cfg;
     b->raster_known = true;
