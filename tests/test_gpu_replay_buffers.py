@@ -56,3 +56,53 @@ def test_two_batches_over_the_same_contexts(engine):
         for r, s in zip(renderers, sc):
             np.testing.assert_array_equal(r.output(), s[size][3])
             assert r.get_error() == 0
+
+
+def test_batch_replay_after_a_resolve_of_other_views(engine):
+    """The batched resolve's descriptors are those of its last call's views."""
+    algs = [oit.OIT_LINKEDLIST, oit.OIT_LOOP64, oit.OIT_LINKEDLIST]
+    cameras = [oit.make_camera(W, H, eye=(x, 0.0, 3.0)) for x in (0.0, 0.7, -0.7)]
+    views, refs = [], []
+    for k, alg in enumerate(algs):
+        v, i, tpo, _ = pu.scene(20, W, H, seed=40 + k)
+        refs.append([pu.render_gpu(alg, W, H, v, i, tpo, sd, 100, **KW)['image'] for sd in cameras])
+        views.append((oit.Renderer(oit.make_state(alg, W, H, **KW)), oit.DeviceMesh(v, i), tpo, 100))
+    batch = oit.Batch(parallel_streams=2)
+
+    def render(which, camera):
+        for k in which:
+            views[k][0].update_scene(cameras[camera])
+        batch.set_views([views[k] for k in which])
+        batch.render()
+        for k in which:
+            np.testing.assert_array_equal(views[k][0].output(), refs[k][camera])
+
+    def resolve(which, camera):
+        for k in which:
+            views[k][0].update_scene(cameras[camera])
+            views[k][0].render_frame(*views[k][1:])
+        batch.set_views([views[k] for k in which])
+        batch.resolve()
+        for k in which:
+            np.testing.assert_array_equal(views[k][0].output(), refs[k][camera])
+
+    render((0, 1), 0)
+    render((0, 1), 1)
+    resolve((2,), 0)
+    render((0, 1), 2)
+    render((0, 1), 0)
+    resolve((0, 1, 2), 1)
+    render((0, 1), 0)
+
+
+def test_batch_with_a_context_made_anew(engine):
+    """A destroyed context's successor, at the same address perhaps, is another view."""
+    s = scenes(oit.OIT_LOOP64, 60)
+    batch = oit.Batch(parallel_streams=2)
+    for n in range(4):
+        with oit.Renderer(oit.make_state(oit.OIT_LOOP64, W, H, **KW)) as r:
+            r.update_scene(s[0][2])
+            batch.set_views([(r, s[0][0], s[0][1], 100)])
+            for _ in range(2):
+                batch.render()
+                np.testing.assert_array_equal(r.output(), s[0][3])

@@ -88,6 +88,12 @@ int cuda_status(cudaError_t e, const char* where) {
 }  // namespace
 
 struct oit_context {
+  // (a batch's signatures: a context made where a destroyed one was is another)
+  const uint64_t id = next_id();
+  static uint64_t next_id() {
+    static std::atomic<uint64_t> n{0};
+    return ++n;
+  }
   oit_state st{};
   int msaa = 1, sample_shading = 0, supersample = 1;
   int W = 0, H = 0, RW = 0, RH = 0;
@@ -934,6 +940,7 @@ struct oit_batch {
   cudaGraphExec_t exec = nullptr;
   uint64_t sig = 0;
   uint64_t moves = 0;  // the views' buffer_moves() at the graph's capture
+  uint64_t graph_rsig = 0;  // rsig at the graph's capture
   uint64_t graph_launches = 0;
   std::vector<oit_context*> ctxs;
   std::vector<bool> opaque_valid;
@@ -1050,11 +1057,13 @@ int batch_prepare_resolve(oit_batch* b, const oit_view_frame* views, uint32_t n)
   for (uint32_t i = 0; i < n; ++i) {
     if (!views[i].ctx->batch_resolvable()) continue;
     ++count;
-    for (uint64_t x : {(uint64_t)(uintptr_t)views[i].ctx, (uint64_t)(uintptr_t)views[i].out_rgba8_device})
+    for (uint64_t x : {views[i].ctx->id, (uint64_t)(uintptr_t)views[i].out_rgba8_device})
       sig = (sig ^ x) * 1099511628211ull;
   }
   sig ^= count;
   if (sig == b->rsig) return OIT_OK;
+  // work under way may read the descriptors that are replaced
+  OIT_TRY_CUDA(cudaDeviceSynchronize(), "sync");
   b->rsig = 0;
   b->r_tuned = false;
   b->r_share = 1.0f;
@@ -1690,10 +1699,9 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
     for (uint32_t j = 0; j < i; ++j)
       if (views[j].ctx == v.ctx) return OIT_ERR_INVALID_ARGUMENT;  // one frame per context
     const oit::MeshRef m = view_mesh(v);
-    const uint64_t parts[] = {(uint64_t)(uintptr_t)v.ctx, (uint64_t)(uintptr_t)m.vertices,
-                              (uint64_t)(uintptr_t)m.indices, (uint64_t)(uintptr_t)m.instances, m.num_triangles,
-                              view_tpo(v), (uint64_t)v.percent_transparent,
-                              (uint64_t)(uintptr_t)v.out_rgba8_device};
+    const uint64_t parts[] = {v.ctx->id, (uint64_t)(uintptr_t)m.vertices, (uint64_t)(uintptr_t)m.indices,
+                              (uint64_t)(uintptr_t)m.instances, m.num_triangles, view_tpo(v),
+                              (uint64_t)v.percent_transparent, (uint64_t)(uintptr_t)v.out_rgba8_device};
     for (uint64_t x : parts) sig = (sig ^ x) * 1099511628211ull;
   }
   sig ^= n;
@@ -1704,7 +1712,7 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
   };
   bool fit = true;
   for (uint32_t i = 0; i < n; ++i) fit = views[i].ctx->graph_bins_fit() && fit;
-  if (!fit || sig != b->sig || moves() != b->moves) b->drop();
+  if (!fit || sig != b->sig || moves() != b->moves || b->rsig != b->graph_rsig) b->drop();
   if (!b->exec) {
     // plain frames, one view after the other, size every buffer (and time
     // each view for the longest-first lane order); views the batched resolve
@@ -1801,6 +1809,7 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
     b->exec = best;
     b->sig = sig;
     b->moves = moves();
+    b->graph_rsig = b->rsig;
     b->graph_launches = best_launches;
     b->raster_cfg = best_cfg;
     b->raster_known = true;
