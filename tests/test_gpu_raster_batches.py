@@ -142,3 +142,41 @@ def test_sort_chunks(engine, n):
     g = pu.render_gpu(oit.OIT_LOOP64, W, H, v, i, 1, scene_data(), 100, **kw)
     o = pu.render_oracle(oit.OIT_LOOP64, W, H, v, i, 1, scene_data(), 100, **kw)
     pu.check_pair(oit.OIT_LOOP64, g, o, W, H, L)
+
+
+@pytest.mark.parametrize('aa', [oit.OIT_AA_NONE, oit.OIT_AA_MSAA_4X, oit.OIT_AA_MSAA_8X, oit.OIT_AA_SSAA_8X])
+@pytest.mark.parametrize('alg', [oit.OIT_LINKEDLIST, oit.OIT_SPINLOCK, oit.OIT_WEIGHTED])
+@pytest.mark.parametrize('W,H', [(128, 96), (101, 83)])
+def test_large_triangles(engine, alg, aa, W, H):
+    """Triangles wider than 64 pixels: quads whose edges run along pixel and
+    micro-tile borders, through pixel centres and just beside them, slivers
+    across the frame, the same quad twice (the first one stays), half of them
+    opaque, with small ones between them."""
+    n, L = 48, 8
+    rng = np.random.default_rng(W)
+    v = np.zeros((n, 2, 3, 10), np.float32)
+    corner = np.array([[0, 0], [1, 0], [1, 1], [0, 1]])
+    for k in range(n):
+        if k % 8 == 7:  # small
+            at, size = rng.uniform(0, 1, 2) * (W, H), rng.uniform(1, 12, 2)
+        else:
+            size = rng.choice([8, 4, 1, 0.5, 1 / 256]) * rng.integers(-3, 4, 2) + (W, H) - rng.integers(0, 24, 2)
+            at = np.floor(rng.uniform(-16, 24, 2)) + rng.choice([0.0, 0.5, 0.5 + 1 / 256, 3 / 16])
+        quad = at + corner * size
+        if k % 5 == 4:
+            quad[2] = quad[0] + rng.uniform(-1, 1, 2)  # a sliver and its back
+        z = rng.uniform(0.05, 0.95, 4)
+        v[k, :, :, :2] = (quad / (W, H) * 2 - 1)[[[0, 1, 2], [0, 2, 3]]]
+        v[k, :, :, 2] = z[[[0, 1, 2], [0, 2, 3]]]
+        if k % 12 == 11:
+            v[k] = v[k - 2]  # equal depths
+    v[:, :, :, 3:6] = rng.normal(size=(n, 1, 1, 3))
+    v[:, :, :, 6:] = rng.random((n, 1, 1, 4))
+    v[:, :, :, 0] *= rng.choice([1, -1], (n, 1, 1))  # both windings, of which opaque ones keep one
+    v, i = v.reshape(-1, 10), np.arange(6 * n, dtype=np.uint32).reshape(-1, 3)
+    order = rng.permutation(n)
+    i = i.reshape(n, 2, 3)[order].reshape(-1, 3)
+    kw = dict(oit_layers=L, nodes_per_pixel=200, aa_type=aa, weighted_precision=oit.OIT_WEIGHTED_FP32)
+    g = pu.render_gpu(alg, W, H, v, i, 2, scene_data(), 50, **kw)
+    o = pu.render_oracle(alg, W, H, v, i, 2, scene_data(), 50, **kw)
+    pu.check_pair(alg, g, o, W, H, L, aa)
