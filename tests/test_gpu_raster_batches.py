@@ -1,8 +1,9 @@
 """The tile raster's batch edges: a warp processes the triangles that touch its
-pixels 32 at a time and queues their fragments 64 at a time, so stacks of
-triangles around those counts, over frames that end inside a tile, a micro-tile
-and a pixel group, against the oracle. Small triangles and ones wider than 64
-pixels (whose edge functions need 64 bits) alternate."""
+pixels 32 at a time and queues their fragments 64 (with several samples a
+lane, 96) at a time, so stacks of triangles around those counts, over frames
+that end inside a tile, a micro-tile and a pixel group, against the oracle.
+Small triangles and ones wider than 64 pixels (whose edge functions need 64
+bits) alternate."""
 import numpy as np
 import pytest
 

@@ -226,15 +226,25 @@ struct oit_context {
     return (alg() == oit::Alg::LinkedList || alg() == oit::Alg::Loop64) && st.record_format == OIT_RECORD_RGBA8 &&
            S == 1 && ssn == 1 && supersample == 1 && !(st.flags & OIT_FLAG_LINEAR_OUTPUT);
   }
-  // Tiles of a frame up to which its rasters take them by list length (the
-  // largest such frame measured, 3645 tiles, is 10% faster; one of 8160 2%
-  // slower); the views of a batch fill the GPU together and keep tile order.
+  // Tiles of a frame up to which its rasters take them by list length: a warp
+  // waits for two more loads and neighbouring tiles no longer run together, but
+  // the frame does not end with its longest lists. Replayed frames of 600
+  // spheres (Loop32: 300) with it against without: 260 to 768 tiles 1-4% slower
+  // (Loop32 with 4x sample shading 2-3% faster), 1200 equal or up to 7% faster,
+  // 1600 to 3645 2-12% faster (that Loop32 11% slower at 3645), 4096 linked list
+  // 1% faster and the others 1-3% slower, 8160 linked list 2% faster and the
+  // others 1-4% slower. The views of a batch fill the GPU together and keep tile
+  // order.
   static constexpr int kOrderMaxTiles = 4096;
   // Triangles of a draw from which the setup tests which micro-tiles a triangle
-  // covers: it costs the setup kernel a microsecond whatever their number (a
-  // staged 948x592 frame of 11,000 triangles 75.7 -> 79.1 us) and spares the
-  // raster a third of its work (linked list 640x480, 245,760 triangles, 107 ->
-  // 103 us; WBOIT 3840x2160, 15.7 million, 2.90 -> 2.69 ms).
+  // covers. The test is work per triangle (3 us of a staged frame of 11,000, 147
+  // us of WBOIT 3840x2160 with 15.7 million) and spares the binning and the
+  // rasters the (triangle, micro-tile) pairs that share no pixel, half of them
+  // where triangles are small. 948x592 frames of spheres, with it against
+  // without: at 7,680 and 16,320 triangles equal within 2 us, small or large
+  // ones; small ones 1-9% faster at 32,640, 4-10% at 65,280, 4-9% at 261,120;
+  // larger ones up to 2% slower at 32,640, up to 3% at 65,280, equal at 130,560,
+  // 1% slower to 3% faster at 261,120. WBOIT 3840x2160 2.69 ms with, 2.90 without.
   static constexpr uint32_t kMicroTriangles = 1u << 16;
   size_t order_words() const { return (size_t)2 * oit::kOrderBuckets * (size_t)num_tiles; }
   int lens_stride() const { return (RW + 7) / 8; }
@@ -414,7 +424,7 @@ struct oit_context {
     // 128 chunks, or one per 2048 pairs and a launch between to sum the
     // counts. A frame alone wants every block busy (64K / 512K: linked list
     // 640x480 94 / 98 us, RGBA32F linked list 700x420 2x2 130 / 132, Spinlock
-    // 800x512 147 / 148; smaller ones have few chunks either way); a batch's
+    // 800x512 equal; smaller ones have few chunks either way); a batch's
     // views fill the GPU together and want fewer launches (24 views 3.43 ms at
     // 8M, 3.44 at 1M)
     b.sort_direct_max = in_batch ? (8u << 20) : (1u << 16);
@@ -813,8 +823,8 @@ struct oit_context {
 
   // ---- CUDA graph of a whole frame (OIT_FLAG_CUDA_GRAPH) ----
   bool capturing = false;
-  bool in_batch = false;
-  int32_t debug_held_lock = -1;  // oit_debug_hold_arrival_lock  // binning inside a batch graph, beside other views
+  bool in_batch = false;         // binning inside a batch graph, beside other views
+  int32_t debug_held_lock = -1;  // oit_debug_hold_arrival_lock
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_sig = 0;
   uint64_t graph_moves = 0;  // buffer_moves() at its capture

@@ -75,7 +75,7 @@ struct Bins {
   uint32_t* keys_alt;
   uint32_t* pair_offset;  // [num_triangles + 1]
   uint32_t* scan_tmp;     // pair counts per 512-triangle block, scanned in place, then the scan's scratch
-  uint32_t* hist;         // the radix sort's digit counts per chunk (and the scanned sort's scratch)
+  uint32_t* hist;         // the radix sort's digit counts per chunk
   uint32_t* total;        // [1] number of pairs (device)
   // tiles of each kind by list length, [2][kOrderBuckets][num_tiles], and how
   // many each bucket holds; null: not wanted
@@ -119,8 +119,9 @@ struct RasterParams {
   const uint32_t* order_count;
   const uint32_t* tile_tris;
   // the sorted pair keys beside tile_tris: tile id (bits 0-23) and the 8x4
-  // micro-tiles of the tile that the triangle's bbox overlaps (bit 24 + k for
-  // micro-tile k = 2 * row + column)
+  // micro-tiles of the tile that the triangle's bbox overlaps, or, tested by the
+  // setup (SetupParams::micro), that it may cover (bit 24 + k for micro-tile
+  // k = 2 * row + column)
   const uint32_t* tile_keys;
   const uint2* bbox;
   const void* setup;

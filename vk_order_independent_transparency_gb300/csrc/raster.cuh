@@ -249,9 +249,10 @@ struct Loop64Policy {
 // fragment, and blend every farther fragment into the target, in order. Here
 // pass 0 keeps depths and colours together; only a warp of which a pixel has
 // dropped a fragment, and only with tail blending, walks the list again (pass 1)
-// to blend what lies behind the kept depths. Against two walks of every list:
-// Loop32 1001x563 4x sample shading 327 -> 262 us, 2000 spheres without tail
-// blending 442 -> 342; with it and nearly every warp walking twice, 448 -> 467.
+// to blend what lies behind the kept depths. Loop32 1001x563 4x sample shading
+// takes 260 us (327 with two walks of every list), dense scenes of 2000 spheres
+// 342 us without tail blending (442) and 467 us with it (448): nearly every warp
+// walks twice there, and shades some fragments twice.
 template <int S>
 struct LoopPolicy {
   static constexpr bool kNodes = false;
@@ -626,8 +627,8 @@ constexpr int kRing = 128;
 // and last = true. A tile's list has a handful of hits per 32 entries (8
 // micro-tiles, triangles of a few pixels), so collecting them first fills the
 // lanes of every later step. chunk is warp-uniform.
-// The test is the 8x4 micro-tile's bit in the pair's sorted key (the binning
-// wrote the bbox's micro-tile overlap there); a warp with fewer pixels than
+// The test is the 8x4 micro-tile's bit in the pair's sorted key (those that the
+// bbox overlaps, or that the setup found covered); a warp with fewer pixels than
 // that (Fine) also tests the bbox. List entries of triangles >= limit are
 // skipped (the second half of a near-clipped triangle t, record num_tris + t,
 // counts as triangle t). With `ident` (an overflowed draw's unbinned
@@ -933,12 +934,13 @@ __device__ __forceinline__ int stage_hits(const WarpTile& w, const TriSetup* set
 // fragment, each with the finding of its hit and pixel around it), and 32
 // fragments are shaded at once; what a fragment's algorithm computes from the
 // fragment alone (its weight, its record, its list node) is done by the lane
-// that shaded it. Whole frames with bbox pairs, then with covered pixels: WBOIT
-// 3840x2160, 16384 spheres 4.60 -> 3.32 ms; Interlock 2560x1440 8x MSAA 4.31 ->
-// 3.63 ms; Loop32 1001x563 4x sample shading 522 -> 391 us; Spinlock 800x512
-// 327 -> 288 us; linked list 640x480 156 -> 137 us; 24-view batch 4.78 -> 4.31
-// ms. (With hits processed per 32 list entries and the edge functions evaluated
-// from the vertices: 6.84 ms, 6.30 ms, 738 us, 420 us, 215 us, 6.18 ms.)
+// that shaded it. Whole frames when that was measured, with covered pixels / with
+// bbox pairs / with hits taken per 32 list entries and the edge functions
+// evaluated from the vertices: WBOIT 3840x2160, 16384 spheres 3.32 / 4.60 / 6.84
+// ms; Interlock 2560x1440 8x MSAA 3.63 / 4.31 / 6.30 ms; Loop32 1001x563 4x sample
+// shading 391 / 522 / 738 us; Spinlock 800x512 288 / 327 / 420 us; linked list
+// 640x480 137 / 156 / 215 us; 24-view batch 4.31 / 4.78 / 6.18 ms.
+// Triangles wider than 64 pixels (64-bit edges) are tested pixel by pixel.
 // The warps of a tile work independently (each walks the tile's list for its
 // own micro-tile), so a CTA holds kRasterWarpsPerBlock of them: a CTA's
 // resources are released when its slowest warp is done, and micro-tiles of

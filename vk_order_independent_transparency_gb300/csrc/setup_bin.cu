@@ -72,6 +72,12 @@ __device__ __forceinline__ uint32_t micro_bits(uint32_t micro, int i, int j) {
   return (micro >> (8 * (2 * j + i))) & 0xFFu;
 }
 
+// Area (in 1/256 pixel squared, times four: 1.5 pixels) up to which a triangle's
+// centres are tested. Against never testing them, 948x592 frames of 65,280 small
+// triangles 51.4 us against 55.5 (linked list) and 53.5 (WBOIT), of 261,120 77.3
+// against 78.2 and 71.9 against 74.8; testing every triangle's is within 1%.
+constexpr int kSliverArea = 4 * 98304;
+
 // Coverage of a small triangle (edge functions in 32 bits; E = 2 e + top_left
 // - 1, no E negative: inside, as in the tile rasters). False when it covers no
 // sample of its pixel bbox, as far as that is tested: every sample of at most
@@ -79,8 +85,6 @@ __device__ __forceinline__ uint32_t micro_bits(uint32_t micro, int i, int j) {
 // 8x16 of a sliver. `covered` is then its micro-tiles, without those that
 // lie outside an edge. (With more samples few of them do: Simple 1283x717 4x
 // MSAA 141 -> 138 us for the raster, 22 -> 27 us for its two setups.)
-constexpr int kSliverArea = 4 * 98304;  // 1.5 pixels (in 1/256 pixel squared, four times the area)
-
 template <int S>
 __device__ __forceinline__ bool small_coverage(const int (&X)[3], const int (&Y)[3], int tl, int bx0, int by0, int bx1,
                                                int by1, bool want_micro, uint32_t& covered) {
@@ -760,8 +764,8 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* ke
 // (counts[digit * nchunks + chunk]); the scatter adds the digit's start, the
 // sum of the last ones of the digits before it. A short kernel, bound by its
 // launch and one or two rounds of loads; a scan of the whole array is three of
-// them (Simple 1283x717 4x MSAA, sorting twice, 294 -> 273 us; Spinlock 800x512
-// 155 -> 148; Loop64 1920x1080 286 -> 281).
+// them (Simple 1283x717 4x MSAA, sorting twice, 294 us with that and 278 with
+// this; Spinlock 800x512 155 and 147; Loop64 1920x1080 286 and 281).
 constexpr int kDigitScanItems = 8;
 
 __global__ void __launch_bounds__(kRadixThreads) k_digit_scan(uint32_t* counts, uint32_t nchunks) {
