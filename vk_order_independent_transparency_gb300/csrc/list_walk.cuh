@@ -266,8 +266,8 @@ __device__ __forceinline__ void net_sort(uint32_t (&d)[K], uint32_t (&c)[K]) {
 // depths are distinct, and blended from the column. Returns false, with nothing blended, for a list longer than K or
 // with equal depths (bubbleSort's order then depends on its passes: the
 // caller's full walk runs it).
-template <int K>
-__device__ __forceinline__ bool walk_list_staged(const uint4* pool, uint32_t head, uint32_t cap, uint32_t* sc,
+template <int K, class Fetch>
+__device__ __forceinline__ bool walk_list_staged(const Fetch& fetch, uint32_t head, uint32_t cap, uint32_t* sc,
                                                  uint32_t* sd, float4& sum) {
   constexpr int T = 32;  // the warp's columns: entry i of a lane at [i * 32 + lane]
   uint32_t off = head < cap ? head : 0u;
@@ -275,7 +275,7 @@ __device__ __forceinline__ bool walk_list_staged(const uint4* pool, uint32_t hea
 #pragma unroll 1
   while (off != 0) {
     if (n == K) return false;
-    const WalkNode nd = load_node<false>(pool, off);
+    const WalkNode nd = fetch(off);
     sc[n * T] = nd.c;
     sd[n * T] = nd.d;
     ++n;
