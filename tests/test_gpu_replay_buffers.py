@@ -106,3 +106,44 @@ def test_batch_with_a_context_made_anew(engine):
             for _ in range(2):
                 batch.render()
                 np.testing.assert_array_equal(r.output(), s[0][3])
+
+
+@pytest.mark.parametrize('own', [True, False])
+def test_overflow_of_a_graph_captured_before_another(engine, own):
+    """Bins that a captured frame's scene outgrows are re-sized by its next
+    call, also when the context was captured for another batch since."""
+    import torch
+    alg = oit.OIT_LOOP64
+    small, large = [oit.make_scene(200, seed=9, radius_min=a, radius_max=b) for a, b in ((0.01, 0.02), (0.2, 0.35))]
+    sd = oit.make_camera(W, H)
+    refs = [pu.render_gpu(alg, W, H, *s, sd, 100, **KW)['image'] for s in (small, large)]
+    r = oit.Renderer(oit.make_state(alg, W, H, flags=oit.OIT_FLAG_CUDA_GRAPH, **KW))
+    r.update_scene(sd)
+    mesh, other = [oit.DeviceMesh(small[0], small[1]) for _ in range(2)]
+
+    def batch(m):
+        b = oit.Batch(parallel_streams=2)
+        b.set_views([(r, m, small[2], 100)])
+        return b
+
+    first = None if own else batch(mesh)
+    second = batch(other)
+
+    def frame():
+        if own:
+            r.render_frame(mesh, small[2], 100)
+        else:
+            first.render()
+        return r.output(), r.get_error()
+
+    for _ in range(2):
+        image, error = frame()
+        np.testing.assert_array_equal(image, refs[0])
+    second.render()
+    mesh.vertices.copy_(torch.from_numpy(large[0]))  # the scene grows behind the same pointer
+    errors = []
+    for _ in range(3):
+        image, error = frame()
+        np.testing.assert_array_equal(image, refs[1])
+        errors.append(error)
+    assert errors == [oit.OIT_DEVERR_BIN_OVERFLOW, 0, 0]

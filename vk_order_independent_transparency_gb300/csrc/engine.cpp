@@ -830,7 +830,7 @@ struct oit_context {
   uint64_t graph_moves = 0;  // buffer_moves() at its capture
   uint64_t graph_launches = 0;
   bool graph_opaque_valid = false;
-  std::vector<uint64_t> graph_stats;
+  std::vector<uint64_t> graph_stats;  // pair-count signatures of the draws captured in it
 
   // Graphs are captured and replayed on a stream the context owns (the legacy
   // default stream cannot be captured); events order it after and before the
@@ -855,9 +855,9 @@ struct oit_context {
   // Pair counts copied back by a graph replay become known once their event
   // completes; returns false when a bin outgrew its capacity (the graph that
   // reads these bins must be re-captured).
-  bool graph_bins_fit() {
+  bool bins_fit(const std::vector<uint64_t>& keys) {
     bool fit = true;
-    for (uint64_t k : graph_stats) {
+    for (uint64_t k : keys) {
       PairStat* ps = pair_stat(k);
       if (ps && ps->pending && cudaEventQuery(ps->ev) == cudaSuccess) {
         ps->known = std::max(ps->known, *ps->host_total);
@@ -868,8 +868,8 @@ struct oit_context {
     return fit;
   }
 
-  int after_graph_launch(cudaStream_t s) {
-    for (uint64_t k : graph_stats) {
+  int after_graph_launch(const std::vector<uint64_t>& keys, cudaStream_t s) {
+    for (uint64_t k : keys) {
       PairStat* ps = pair_stat(k);
       if (ps && !ps->pending) {
         OIT_TRY_CUDA(cudaEventRecord(ps->ev, s), "event");
@@ -890,7 +890,7 @@ struct oit_context {
     for (uint64_t v : parts) sig = (sig ^ v) * 1099511628211ull;
     // bins that outgrew their capacity since the capture invalidate the graph,
     // and so do buffers that another draw, or a batch, made grow
-    if (!graph_bins_fit() || graph_moves != buffer_moves()) drop_graph();
+    if (!bins_fit(graph_stats) || graph_moves != buffer_moves()) drop_graph();
     int gr = ensure_graph_stream();
     if (gr != OIT_OK) return gr;
     if (!graph_exec || graph_sig != sig) {
@@ -931,7 +931,7 @@ struct oit_context {
     OIT_TRY_CUDA(cudaEventRecord(graph_out, graph_stream), "event");
     OIT_TRY_CUDA(cudaStreamWaitEvent(s, graph_out, 0), "wait");
     launches += graph_launches;
-    int ar = after_graph_launch(graph_stream);
+    int ar = after_graph_launch(graph_stats, graph_stream);
     if (ar != OIT_OK) return ar;
     opaque_valid = graph_opaque_valid;  // as left by the captured frame
     color_valid = true;
@@ -954,6 +954,7 @@ struct oit_batch {
   uint64_t graph_launches = 0;
   std::vector<oit_context*> ctxs;
   std::vector<bool> opaque_valid;
+  std::vector<std::vector<uint64_t>> stats;  // each view's graph_stats in this graph
 
   // Batched resolve of the views that allow it (oit_context::batch_resolvable),
   // in two parts, linked-list views and Loop64 views, each with its view
@@ -1370,6 +1371,7 @@ int batch_capture(oit_batch* b, const oit_view_frame* views, uint32_t n, cudaStr
   uint64_t nodes = 0;
   b->ctxs.assign(n, nullptr);
   b->opaque_valid.assign(n, false);
+  b->stats.assign(n, {});
   std::vector<uint32_t> order;
   std::vector<size_t> lane;
   batch_lanes(b, n, lane_order, order, lane);
@@ -1378,13 +1380,14 @@ int batch_capture(oit_batch* b, const oit_view_frame* views, uint32_t n, cudaStr
     const oit_view_frame& v = views[i];
     oit_context* c = v.ctx;
     const uint64_t l0 = c->launches;
-    c->graph_stats.clear();
+    b->stats[i].swap(c->graph_stats);  // (the context's own graph keeps its)
     c->capturing = true;
     c->in_batch = true;
     r = c->render_frame_body(view_mesh(v), view_tpo(v), v.percent_transparent, v.out_rgba8_device,
                              b->lanes[lane[i]], !multi_view && !c->batch_resolvable(), !multi_view);
     c->capturing = false;
     c->in_batch = false;
+    b->stats[i].swap(c->graph_stats);
     nodes += c->launches - l0;
     c->launches = l0;
     c->last_stream = s;
@@ -1721,7 +1724,7 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
     return m;
   };
   bool fit = true;
-  for (uint32_t i = 0; i < n; ++i) fit = views[i].ctx->graph_bins_fit() && fit;
+  for (uint32_t i = 0; i < n && sig == b->sig && b->exec; ++i) fit = views[i].ctx->bins_fit(b->stats[i]) && fit;
   if (!fit || sig != b->sig || moves() != b->moves || b->rsig != b->graph_rsig) b->drop();
   if (!b->exec) {
     // plain frames, one view after the other, size every buffer (and time
@@ -1836,7 +1839,7 @@ int oit_batch_render(oit_batch* b, const oit_view_frame* views, uint32_t n, void
   OIT_TRY_CUDA(cudaStreamWaitEvent(s, b->out, 0), "wait");
   for (uint32_t i = 0; i < n; ++i) {
     oit_context* c = b->ctxs[i];
-    int r = c->after_graph_launch(b->stream);
+    int r = c->after_graph_launch(b->stats[i], b->stream);
     if (r != OIT_OK) return r;
     c->launches += 0;
     c->opaque_valid = b->opaque_valid[i];
