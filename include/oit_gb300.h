@@ -308,7 +308,9 @@ int oit_batch_destroy(oit_batch* batch);
 
 /* Renders every view (Sample::onRender per view). The first call with a given
  * set of views renders them one by one (sizing their buffers) and captures the
- * graph; later calls replay it. Ordered after prior work on `stream`. */
+ * graph; later calls replay it, or do this again where another call made a
+ * context's buffers grow, a scene outgrew its bins or oit_batch_resolve was
+ * called with other views. Ordered after prior work on `stream`. */
 int oit_batch_render(oit_batch* batch, const oit_view_frame* views, uint32_t num_views, void* stream);
 
 /* Kernel launches per replay of the batch's graph. */
